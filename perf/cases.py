@@ -217,3 +217,80 @@ def tolerance(case):
         return {"rel": 2e-2, "max": 0.5}   # P in e4m3 (2^-4 a value): another split into tiles rounds other values
     # bf16 outputs and bf16 / fp16 probabilities; the vertical-line indices are whole numbers (a tie may swap a few)
     return {"rel": 6e-3, "max": 0.1, "differ": 1e-3}
+
+
+# ---------------------------------------------------------------------------------------------------------------
+# The same calls in 64 bits, in plain torch: what the quantised cache and the attention over it are by definition.
+
+def _quant64(x, bits):
+    """[..., n, 128] -> the values that the per-token codes and fp16 scales stand for."""
+    qmax = float(2 ** (bits - 1) - 1)
+    scale = (x.float().abs().amax(-1, keepdim=True).clamp_min(1e-5) * (1.0 / torch.tensor(qmax)).to(x.device)).half().double()
+    return (x.double() / scale).round().clamp(-qmax - 1, qmax) * scale
+
+
+def _frozen64(case, g):
+    """[B, hkv, m, 128] keys and values of a layer's cache after freeze, as the codes and rows it holds."""
+    k, v, q = g["k"], g["v"], g["q"]
+    B, hkv, n, R, W = k.shape[0], k.shape[1], k.shape[2], q.shape[1] // k.shape[1], min(case["window"], k.shape[2])
+    kp, vp, kw, vw = k[:, :, :n - W], v[:, :, :n - W], k[:, :, n - W:].double(), v[:, :, n - W:].double()
+    T = _segments(case)[1]
+    kq, vq = _quant64(kp, case["k_bits"]), _quant64(vp, case["v_bits"])
+    if T:
+        tail = q[:, :, -W:].reshape(B, hkv, R, -1, D).mean(dim=2).double().mean(dim=2, keepdim=True)
+        score = (kp[:, :, :n - 2 * W].double() @ tail.transpose(2, 3)).squeeze(3)
+        idx = score.topk(T, dim=-1).indices[..., None].expand(-1, -1, -1, D)
+        kq.scatter_(2, idx, kp.gather(2, idx).double())
+        vq.scatter_(2, idx, vp.gather(2, idx).double())
+    return torch.cat([kq, kw], dim=2), torch.cat([vq, vw], dim=2)
+
+
+def _attend64(q, k, v):
+    B, hq = q.shape[:2]
+    s = q.double().reshape(B, k.shape[1], -1, D) @ k.transpose(2, 3) / math.sqrt(D)
+    return (s.softmax(dim=-1) @ v).reshape(B, hq, 1, D)
+
+
+def exact(case, seed):
+    kind, B, hq, hkv = case["kind"], case["B"], case["hq"], case["hkv"]
+    if kind == "freeze":
+        return None                        # codes, copied rows and indices: whole numbers and bytes
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(seed + 7919)
+    if kind == "decode":
+        g = _inputs(case, seed, n_qry=case["window"])
+        k, v = _frozen64(case, g)
+        if case["staging"]:
+            ks, vs = _rows(gen, B, hkv, case["staging"], D), _rows(gen, B, hkv, case["staging"], D)
+            k, v = torch.cat([k, ks.double()], dim=2), torch.cat([v, vs.double()], dim=2)
+        return _attend64(g["q_decode"], k, v)
+    if kind == "token":
+        rows, out = _rows(gen, case["layers"], B, hq + 2 * hkv, 1, D), []
+        for i in range(case["layers"]):
+            k, v = _frozen64(case, _inputs(case, 1000 * seed + i, n_qry=case["window"]))
+            kn, vn = rows[i, :, hq:hq + hkv].double(), rows[i, :, hq + hkv:].double()
+            out.append(_attend64(rows[i, :, :hq], torch.cat([k, kn], dim=2), torch.cat([v, vn], dim=2)))
+        return torch.stack(out)
+    if kind == "answer":
+        g, t = _inputs(case, seed, n_qry=case["window"]), case["tokens"]
+        q, kn, vn = _rows(gen, t, B, hq, 1, D), _rows(gen, t, B, hkv, 1, D), _rows(gen, t, B, hkv, 1, D)
+        (k, v), out, first = _frozen64(case, g), [], 0
+        for i in range(t):
+            if i + 1 - first == 128:       # the staging buffer is full: its tokens are quantised before this attention
+                ks, vs = torch.cat(list(kn[first:i + 1]), dim=2), torch.cat(list(vn[first:i + 1]), dim=2)
+                k, v, first = torch.cat([k, _quant64(ks, case["k_bits"])], dim=2), torch.cat([v, _quant64(vs, case["v_bits"])], dim=2), i + 1
+            ks, vs = [x.double() for x in kn[first:i + 1]], [x.double() for x in vn[first:i + 1]]
+            out.append(_attend64(q[i], torch.cat([k] + ks, dim=2), torch.cat([v] + vs, dim=2)))
+        return torch.stack(out)
+    g, n, R = _inputs(case, seed), case["n"], hq // hkv
+    out = torch.empty(B, hq, n, D, dtype=torch.float64, device="cuda")
+    at = torch.arange(n, device="cuda")
+    for b in range(B):
+        for h in range(hq):
+            k, v = g["k"][b, h // R].double(), g["v"][b, h // R].double()
+            for i in range(0, n, 4096):
+                j = min(i + 4096, n)
+                s = (g["q"][b, h, i:j].double() / math.sqrt(D)) @ k[:j].T
+                s.masked_fill_(at[None, :j] > at[i:j, None], float("-inf"))
+                out[b, h, i:j] = s.softmax(dim=-1) @ v[:j]
+    return (out, None) if kind == "hybrid" else out

@@ -134,6 +134,14 @@ __device__ __forceinline__ uint32_t pack_e4m3x4(float a, float b, float c, float
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
+// One lane of a converged warp.  A warp whose 32 lanes walk a loop together and elect a lane only for the tensor
+// instructions keeps descriptors and addresses in uniform registers.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
+}
+
 // ------------------------------------------------------------------ device: MMA
 // Shared-memory operand descriptor for a K-major tile whose rows are 128 bytes, 128-byte swizzle:
 // 8-row groups are 1024 bytes apart; the tile base must be 1024-byte aligned.  Stepping along K

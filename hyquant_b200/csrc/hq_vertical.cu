@@ -9,9 +9,10 @@
 // K fragments come straight from global memory as 16-byte loads; the channel
 // axis is permuted consistently on both operands so that no shuffle is needed.
 //
-// Top-k kernel — one CTA per row: 4-pass radix select of the k-th largest key,
-// order-preserving compaction (ties go to the lower index), bitonic sort of
-// the selected (key, ~index) pairs in shared memory.
+// Top-k kernel — latency-bound, one CTA per row (8 to 32 rows of a call): the row's keys are read once, eight loads a
+// thread in flight, and kept in shared memory; three-pass radix select of the k-th largest key with a scan over the
+// bins, order-preserving compaction (ties go to the lower index; it is also the ascending list), bitonic sort of the
+// selected (key, ~index) pairs, the short distances inside warps.
 #include "hq_common.cuh"
 
 namespace hq {
@@ -19,25 +20,74 @@ namespace hq {
 // ------------------------------------------------------------------ pooling
 // `group` > 1: output head h is the mean of the input heads h group .. h group + group - 1, taken per token and rounded
 // to the input dtype (what a 16-bit mean over the head axis gives) before the tokens are pooled.
+//
+// Latency-bound: a few hundred KB in all.  One block per (output head, 16 channels): 256 threads fetch 128 tokens of
+// all the group's heads at once, 16 bytes a load where the rows are aligned, and leave the per-token means in shared
+// memory, where one thread per channel adds them up in token order (the order of the sum decides ties of the
+// selection, so it stays).  One thread per channel with a dependent load per token and head took 93 us for 8 kv-heads
+// x 4 heads x 128 tokens.
+constexpr int kPoolRows = 128;    // tokens per trip
+constexpr int kPoolCh = 16;       // channels per block
+constexpr int kPoolThreads = kPoolRows * kPoolCh / 8;
+
 template <typename T>
-__global__ void pool_query_kernel(const T* __restrict__ q, int64_t sb, int64_t sh, int64_t sn, int H_Q, int n_q,
-                                  int tail_len, int round_mode /*-1 none, else dtype*/, int group, int group_dtype,
-                                  float* __restrict__ pooled) {
-  const int bh = blockIdx.x, b = bh / H_Q, h = bh - b * H_Q, d = threadIdx.x;
-  const T* base = q + b * sb + (int64_t)h * group * sh + (int64_t)(n_q - tail_len) * sn + d;
-  float acc = 0.f;
-  if (group <= 1) {
-    for (int i = 0; i < tail_len; ++i) acc += load_as_float<T>(base + i * sn);
+__device__ __forceinline__ void load8(const T* p, bool vec, float (&v)[8]) {
+  if (vec) {
+    const uint4 raw = __ldg(reinterpret_cast<const uint4*>(p));
+    const T* e = reinterpret_cast<const T*>(&raw);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = load_as_float<T>(e + j);
   } else {
-    for (int i = 0; i < tail_len; ++i) {
-      float s = 0.f;
-      for (int r = 0; r < group; ++r) s += load_as_float<T>(base + r * sh + i * sn);
-      acc += out_round(s / (float)group, group_dtype);
-    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = load_as_float<T>(p + j);
   }
-  float m = acc / (float)tail_len;
-  if (round_mode >= 0) m = out_round(m, round_mode);
-  pooled[(int64_t)bh * 128 + d] = m;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kPoolThreads)
+pool_query_kernel(const T* __restrict__ q, int64_t sb, int64_t sh, int64_t sn, int H_Q, int n_q,
+                  int tail_len, int round_mode /*-1 none, else dtype*/, int group, int group_dtype,
+                  int vec /* rows are 16-byte aligned */, float* __restrict__ pooled) {
+  __shared__ float s_mean[kPoolRows][kPoolCh + 1];
+  const int bh = blockIdx.x, b = bh / H_Q, h = bh - b * H_Q, d0 = blockIdx.y * kPoolCh;
+  const int tid = threadIdx.x, r0 = tid >> 1, c = (tid & 1) * 8;
+  const T* base = q + b * sb + (int64_t)h * group * sh + (int64_t)(n_q - tail_len) * sn + d0 + c;
+  float acc = 0.f;
+  for (int i0 = 0; i0 < tail_len; i0 += kPoolRows) {
+    const int i = i0 + r0;
+    if (i < tail_len) {
+      float m[8];
+      if (group <= 1) {
+        load8<T>(base + (int64_t)i * sn, vec, m);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) m[j] = 0.f;
+#pragma unroll 4
+        for (int r = 0; r < group; ++r) {
+          float v[8];
+          load8<T>(base + r * sh + (int64_t)i * sn, vec, v);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) m[j] += v[j];
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) m[j] = out_round(m[j] / (float)group, group_dtype);
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) s_mean[r0][c + j] = m[j];
+    }
+    __syncthreads();
+    if (tid < kPoolCh) {
+      const int rows = min(kPoolRows, tail_len - i0);
+#pragma unroll 8
+      for (int r = 0; r < rows; ++r) acc += s_mean[r][tid];
+    }
+    __syncthreads();
+  }
+  if (tid < kPoolCh) {
+    float m = acc / (float)tail_len;
+    if (round_mode >= 0) m = out_round(m, round_mode);
+    pooled[(int64_t)bh * 128 + d0 + tid] = m;
+  }
 }
 
 // ------------------------------------------------------------------ scores
@@ -175,78 +225,136 @@ __device__ __forceinline__ int block_exclusive_scan(int v, int* warp_sums, int& 
   return warp_sums[warp] + inc - v;
 }
 
+constexpr int kTopkBins = 2048;
+
+// 64 entries per warp (lane l: base + l and base + 32 + l): the compare-exchange steps of a bitonic stage `size` whose
+// distance is at most `first` (32 or less), without leaving registers
+__device__ __forceinline__ void bitonic_in_warp(unsigned long long& a, unsigned long long& c, int base, int lane, int size, int first) {
+  if (first >= 32) {
+    const bool desc = ((base + lane) & size) == 0;
+    if ((a < c) == desc) { const unsigned long long x = a; a = c; c = x; }
+    first = 16;
+  }
+  const bool da = ((base + lane) & size) == 0, dc = ((base + 32 + lane) & size) == 0;
+  for (int strd = first; strd > 0; strd >>= 1) {
+    const unsigned long long pa = __shfl_xor_sync(0xffffffffu, a, strd), pc = __shfl_xor_sync(0xffffffffu, c, strd);
+    const bool lower = (lane & strd) == 0;
+    a = ((a > pa) == (lower == da)) ? a : pa;
+    c = ((c > pc) == (lower == dc)) ? c : pc;
+  }
+}
+
+// kCached: the row's keys stay in shared memory after the first pass (rows of up to some 50 thousand candidates);
+// longer rows read them again from L2.
+template <bool kCached>
 __global__ void __launch_bounds__(kTopkThreads)
 topk_kernel(const float* __restrict__ scores, int64_t stride, int n, int k, int kpad,
             int64_t* __restrict__ idx_desc, int32_t* __restrict__ idx_asc) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   unsigned long long* sel = reinterpret_cast<unsigned long long*>(smem_raw);   // [kpad]
-  __shared__ int hist[256];
+  int* hist = reinterpret_cast<int*>(sel + kpad);                              // [kTopkBins]
+  uint32_t* keys = reinterpret_cast<uint32_t*>(hist + kTopkBins);              // [n] if kCached
   __shared__ int warp_sums[33];
-  __shared__ uint32_t s_prefix;
+  __shared__ uint32_t s_bin;
   __shared__ int s_remaining;
-  __shared__ int s_count;
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const float* row = scores + (int64_t)blockIdx.x * stride;
+  auto key_at = [&](int i) -> uint32_t { return kCached ? keys[i] : orderable(__ldg(row + i)); };
 
-  // ---- radix select: find key T of the k-th largest element
+  // ---- radix select: find key T of the k-th largest element (digits of 11, 11 and 10 bits)
   uint32_t prefix = 0, mask = 0;
   int remaining = k;   // rank (1-based from the top) within the current candidate set
-  for (int pass = 0; pass < 4; ++pass) {
-    const int shift = 24 - 8 * pass;
-    if (tid < 256) hist[tid] = 0;
+#pragma unroll 1
+  for (int pass = 0; pass < 3; ++pass) {
+    const int shift = pass == 0 ? 21 : pass == 1 ? 10 : 0;
+    const uint32_t digits = pass == 2 ? 1023u : 2047u;
+    for (int x = tid; x < kTopkBins; x += kTopkThreads) hist[x] = 0;
     __syncthreads();
-    for (int i = tid; i < n; i += kTopkThreads) {
-      const uint32_t key = orderable(__ldg(row + i));
-      if ((key & mask) == prefix) atomicAdd(&hist[(key >> shift) & 0xFF], 1);
-    }
-    __syncthreads();
-    if (tid == 0) {
-      int rem = remaining, b = 255;
-      for (; b > 0; --b) {
-        if (hist[b] >= rem) break;
-        rem -= hist[b];
+    for (int i0 = tid; i0 < n; i0 += 8 * kTopkThreads) {
+      uint32_t key[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int i = i0 + j * kTopkThreads;
+        key[j] = i < n ? ((kCached && pass > 0) ? keys[i] : orderable(__ldg(row + i))) : 0u;
       }
-      s_prefix = prefix | ((uint32_t)b << shift);
-      s_remaining = rem;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int i = i0 + j * kTopkThreads;
+        if (i < n) {
+          if (kCached && pass == 0) keys[i] = key[j];
+          if ((key[j] & mask) == prefix) atomicAdd(&hist[(key[j] >> shift) & digits], 1);
+        }
+      }
     }
     __syncthreads();
-    prefix = s_prefix;
-    remaining = s_remaining;
-    mask |= 0xFFu << shift;
+    // the digit that holds the wanted rank: thread t has the bins kTopkBins - 1 - 2 t and the one below it
+    const int h0 = hist[kTopkBins - 1 - 2 * tid], h1 = hist[kTopkBins - 2 - 2 * tid];
+    int total;
+    const int above = block_exclusive_scan(h0 + h1, warp_sums, total);
+    if (above < remaining && remaining <= above + h0 + h1) {
+      const bool first = remaining <= above + h0;
+      s_bin = (uint32_t)(kTopkBins - 1 - 2 * tid - (first ? 0 : 1));
+      s_remaining = remaining - above - (first ? 0 : h0);
+    }
     __syncthreads();
+    prefix |= s_bin << shift;
+    remaining = s_remaining;
+    mask |= digits << shift;
   }
   const uint32_t T = prefix;        // threshold key
   const int need_eq = remaining;    // how many elements equal to T to take (lowest indices first)
 
-  // ---- order-preserving compaction into sel[]
-  if (tid == 0) s_count = 0;
-  __syncthreads();
-  int eq_taken = 0;   // running number of == T elements seen in earlier tiles (block-uniform)
-  int out_base = 0;   // running number of selected elements
-  for (int base = 0; base < n; base += kTopkThreads) {
-    const int i = base + tid;
-    uint32_t key = 0;
-    int is_gt = 0, is_eq = 0;
-    if (i < n) {
-      key = orderable(__ldg(row + i));
-      is_gt = key > T;
-      is_eq = key == T;
-    }
-    int eq_total;
-    const int eq_rank = block_exclusive_scan(is_eq, warp_sums, eq_total);
-    const int take = is_gt || (is_eq && (eq_taken + eq_rank) < need_eq);
-    int take_total;
-    const int pos = block_exclusive_scan(take, warp_sums, take_total);
-    if (take) sel[out_base + pos] = ((unsigned long long)key << 32) | (uint32_t)(~(uint32_t)i);
-    eq_taken += eq_total;
-    out_base += take_total;
+  // ---- order-preserving compaction into sel[]: warp w owns one contiguous range of the row, counts what it has and
+  // writes once the warps before it are known; the order of the list is the ascending index list
+  const int seg = ((n + 31) / 32 + 31) & ~31;
+  const int s0 = min(warp * seg, n), s1 = min(s0 + seg, n);
+  int gt = 0, eq = 0;
+  for (int i = s0 + lane; i < s1; i += 32) {
+    const uint32_t key = key_at(i);
+    gt += key > T;
+    eq += key == T;
   }
-  for (int i = out_base + tid; i < kpad; i += kTopkThreads) sel[i] = 0ull;   // smaller than any real entry
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    gt += __shfl_xor_sync(0xffffffffu, gt, o);
+    eq += __shfl_xor_sync(0xffffffffu, eq, o);
+  }
+  int total;
+  const int eq_scan = block_exclusive_scan(lane == 0 ? eq : 0, warp_sums, total);
+  int eq_seen = __shfl_sync(0xffffffffu, eq_scan, 0);           // == T elements of the warps before
+  const int mine = gt + max(0, min(eq, need_eq - eq_seen));
+  const int out_scan = block_exclusive_scan(lane == 0 ? mine : 0, warp_sums, total);
+  int out_pos = __shfl_sync(0xffffffffu, out_scan, 0);
+  if (mine > 0) {
+    const uint32_t lt = (1u << lane) - 1u;
+    for (int i0 = s0; i0 < s1; i0 += 32) {
+      const int i = i0 + lane;
+      const uint32_t key = i < s1 ? key_at(i) : 0u;
+      const bool is_eq = i < s1 && key == T;
+      const uint32_t eqs = __ballot_sync(0xffffffffu, is_eq);
+      const bool take = i < s1 && (key > T || (is_eq && eq_seen + __popc(eqs & lt) < need_eq));
+      const uint32_t takes = __ballot_sync(0xffffffffu, take);
+      if (take) {
+        const int pos = out_pos + __popc(takes & lt);
+        sel[pos] = ((unsigned long long)key << 32) | (uint32_t)(~(uint32_t)i);
+        if (idx_asc) idx_asc[(int64_t)blockIdx.x * k + pos] = i;
+      }
+      eq_seen += __popc(eqs);
+      out_pos += __popc(takes);
+    }
+  }
+  for (int i = k + tid; i < kpad; i += kTopkThreads) sel[i] = 0ull;   // smaller than any real entry
   __syncthreads();
 
-  // ---- bitonic sort, descending
-  for (int size = 2; size <= kpad; size <<= 1) {
-    for (int strd = size >> 1; strd > 0; strd >>= 1) {
+  // ---- bitonic sort, descending: distances of 64 and more through shared memory, the rest inside warps
+  for (int base = warp * 64; base < kpad; base += (kTopkThreads / 32) * 64) {
+    unsigned long long a = sel[base + lane], c = sel[base + 32 + lane];
+    for (int size = 2; size <= 64; size <<= 1) bitonic_in_warp(a, c, base, lane, size, size >> 1);
+    sel[base + lane] = a; sel[base + 32 + lane] = c;
+  }
+  __syncthreads();
+  for (int size = 128; size <= kpad; size <<= 1) {
+    for (int strd = size >> 1; strd >= 64; strd >>= 1) {
       for (int x = tid; x < (kpad >> 1); x += kTopkThreads) {
         const int lo = 2 * x - (x & (strd - 1));
         const int hi = lo + strd;
@@ -256,28 +364,15 @@ topk_kernel(const float* __restrict__ scores, int64_t stride, int n, int k, int 
       }
       __syncthreads();
     }
+    for (int base = warp * 64; base < kpad; base += (kTopkThreads / 32) * 64) {
+      unsigned long long a = sel[base + lane], c = sel[base + 32 + lane];
+      bitonic_in_warp(a, c, base, lane, size, 32);
+      sel[base + lane] = a; sel[base + 32 + lane] = c;
+    }
+    __syncthreads();
   }
   for (int i = tid; i < k; i += kTopkThreads)
     idx_desc[(int64_t)blockIdx.x * k + i] = (int64_t)(~(uint32_t)(sel[i] & 0xFFFFFFFFull));
-  if (idx_asc == nullptr) return;
-  __syncthreads();
-  // ---- the same set in ascending position: sort the indices
-  uint32_t* ids = reinterpret_cast<uint32_t*>(smem_raw) + 2 * kpad;   // after sel[]
-  for (int i = tid; i < kpad; i += kTopkThreads) ids[i] = i < k ? ~(uint32_t)(sel[i] & 0xFFFFFFFFull) : 0xFFFFFFFFu;
-  __syncthreads();
-  for (int size = 2; size <= kpad; size <<= 1) {
-    for (int strd = size >> 1; strd > 0; strd >>= 1) {
-      for (int x = tid; x < (kpad >> 1); x += kTopkThreads) {
-        const int lo = 2 * x - (x & (strd - 1));
-        const int hi = lo + strd;
-        const bool asc = ((lo & size) == 0);
-        const uint32_t a = ids[lo], b2 = ids[hi];
-        if ((a > b2) == asc) { ids[lo] = b2; ids[hi] = a; }
-      }
-      __syncthreads();
-    }
-  }
-  for (int i = tid; i < k; i += kTopkThreads) idx_asc[(int64_t)blockIdx.x * k + i] = (int32_t)ids[i];
 }
 
 }  // namespace hq
@@ -301,12 +396,14 @@ static int vertical_scores_impl(const void* q, int io_dtype, int64_t q_stride_b,
              "hq_vertical_scores: key rows must be 16-byte aligned");
   cudaStream_t st = (cudaStream_t)stream;
   const int rm = round_mean ? io_dtype : -1;
+  const int vec = aligned16(q) && q_stride_b % 8 == 0 && q_stride_h % 8 == 0 && q_stride_n % 8 == 0;
+  const dim3 pgrid((unsigned)(B * H_Q), 128 / kPoolCh);
   if (io_dtype == HQ_BF16)
-    pool_query_kernel<__nv_bfloat16><<<B * H_Q, 128, 0, st>>>((const __nv_bfloat16*)q, q_stride_b, q_stride_h, q_stride_n, H_Q,
-                                                              n_q, tail_len, rm, group, io_dtype, pooled);
+    pool_query_kernel<__nv_bfloat16><<<pgrid, kPoolThreads, 0, st>>>((const __nv_bfloat16*)q, q_stride_b, q_stride_h, q_stride_n, H_Q,
+                                                                     n_q, tail_len, rm, group, io_dtype, vec, pooled);
   else
-    pool_query_kernel<__half><<<B * H_Q, 128, 0, st>>>((const __half*)q, q_stride_b, q_stride_h, q_stride_n, H_Q, n_q,
-                                                       tail_len, rm, group, io_dtype, pooled);
+    pool_query_kernel<__half><<<pgrid, kPoolThreads, 0, st>>>((const __half*)q, q_stride_b, q_stride_h, q_stride_n, H_Q, n_q,
+                                                              tail_len, rm, group, io_dtype, vec, pooled);
   HQ_CUDA(cudaGetLastError());
   const int tiles = (n_cand + 15) / 16;
   int chunks = (2 * sm_count() + B * H_KV - 1) / (B * H_KV);
@@ -358,17 +455,22 @@ extern "C" int hq_topk(const float* scores, int64_t scores_stride, int rows, int
   HQ_REQUIRE(k <= n, HQ_ERR_INVALID, "hq_topk: k %d > n %d", k, n);
   HQ_REQUIRE(k <= kTopkMaxK, HQ_ERR_UNSUPPORTED, "hq_topk: k %d > %d", k, kTopkMaxK);
   HQ_REQUIRE(scores && idx_desc, HQ_ERR_INVALID, "hq_topk: null pointer");
-  int kpad = 2;
+  int kpad = 64;
   while (kpad < k) kpad <<= 1;
-  const size_t smem = (size_t)kpad * 8 + (size_t)kpad * 4;
+  constexpr size_t kMaxSmem = 224 * 1024;
+  const size_t need = (size_t)kpad * 8 + kTopkBins * 4, with_keys = need + (size_t)n * 4;
   static thread_local int attr_dev = -1;
   int dev = 0;
   HQ_CUDA(cudaGetDevice(&dev));
   if (attr_dev != dev) {
-    HQ_CUDA(cudaFuncSetAttribute(topk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTopkMaxK * 12));
+    HQ_CUDA(cudaFuncSetAttribute(topk_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem));
+    HQ_CUDA(cudaFuncSetAttribute(topk_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem));
     attr_dev = dev;
   }
-  topk_kernel<<<rows, kTopkThreads, smem, (cudaStream_t)stream>>>(scores, scores_stride, n, k, kpad, idx_desc, idx_asc);
+  if (with_keys <= kMaxSmem)
+    topk_kernel<true><<<rows, kTopkThreads, with_keys, (cudaStream_t)stream>>>(scores, scores_stride, n, k, kpad, idx_desc, idx_asc);
+  else
+    topk_kernel<false><<<rows, kTopkThreads, need, (cudaStream_t)stream>>>(scores, scores_stride, n, k, kpad, idx_desc, idx_asc);
   HQ_CUDA(cudaGetLastError());
   return HQ_OK;
 }

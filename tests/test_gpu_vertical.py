@@ -87,6 +87,44 @@ def test_topk_exact_with_ties(n, k):
     assert np.array_equal(asc.cpu().numpy(), np.sort(ref, axis=-1))
 
 
+@pytest.mark.parametrize("n,k", [(31, 5), (64, 64), (65, 64), (1025, 129), (53000, 2650), (56000, 100), (56300, 100), (60000, 16384)])
+def test_topk_edges_of_the_kept_row_and_the_warp_ranges(n, k):
+    """Rows that just fit the shared-memory copy of the keys and rows that do not, ranges of warps that are empty, lists
+    around the 64 entries a warp sorts by itself; infinities and a row of one value."""
+    rng = np.random.Generator(np.random.PCG64(7 * n + k))
+    s = rng.standard_normal((4, n), dtype=np.float32)
+    s[1] = 0.25
+    s[2, rng.integers(0, n, size=max(1, n // 3))] = -np.inf
+    s[3, rng.integers(0, n, size=3)] = np.inf
+    idx, asc = hq.topk_indices(torch.from_numpy(s).to(DEV), k, want_ascending=True)
+    ref = orc.topk_desc(s, k)
+    assert np.array_equal(idx.cpu().numpy(), ref)
+    assert np.array_equal(asc.cpu().numpy(), np.sort(ref, axis=-1))
+
+
+@pytest.mark.parametrize("tail,R,offset", [(1, 1, 0), (127, 4, 0), (128, 7, 0), (129, 4, 8), (300, 2, 4), (256, 1, 4)])
+def test_pooled_query_is_the_sum_in_token_order(tail, R, offset):
+    """The pooled query decides ties of the selection: the fp32 sum over the tokens in their order, bit for bit, from
+    aligned and from unaligned rows.  A key row that is a unit vector reads one channel back."""
+    g = torch.Generator(device=DEV); g.manual_seed(tail + R)
+    q = torch.randn(1, 2 * R, tail, 128 + offset, generator=g, device=DEV, dtype=torch.float32).to(torch.bfloat16)[..., offset:]
+    k = torch.eye(128, device=DEV, dtype=torch.bfloat16).expand(1, 2, 128, 128).contiguous()
+    keys = torch.cat([k, torch.zeros(1, 2, tail, 128, device=DEV, dtype=torch.bfloat16)], dim=2)
+    got = hq.vertical_scores(q, keys, tail, 1, group_mean=R)
+    m = q.float().reshape(1, 2, R, tail, 128).cpu().numpy()
+    s = np.zeros((1, 2, tail, 128), np.float32)
+    for r in range(R):
+        s += m[:, :, r]
+    if R > 1:
+        s = orc.bf16_round(s / np.float32(R))
+    acc = np.zeros((1, 2, 128), np.float32)
+    for i in range(tail):
+        acc += s[:, :, i]
+    want = acc / np.float32(tail)
+    # the scores split the mean into two bf16 parts: 2^-16 of the value at most
+    assert np.all(np.abs(got.cpu().numpy() - want) <= 2.0 ** -16 * np.abs(want))
+
+
 def test_topk_limits():
     s = torch.zeros(1, 40000, device=DEV)
     with pytest.raises(hq.HyQuantError):

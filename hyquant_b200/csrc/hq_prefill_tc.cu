@@ -419,7 +419,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap mQi, const __grid_constant
     const uint32_t colS = kColS + 128 * h, colO = kColO + 128 * h;
     const int n_rest = plan.n_rest, n_vert = plan.nvert(h), nvh = h ? nv1 : nv0;
     // rows past N compute on a token scale, so that a masked column (-inf) times the scale stays -inf
-    const float qs = (row < p.N && n_tiles > 0) ? p.q_scale[bhq * p.Npad + row] : 1e-30f;
+    const float qs = (row < p.N && n_tiles > 0 && n_rest > 0) ? p.q_scale[bhq * p.Npad + row] : 1e-30f;
     float m_ref = row < p.N ? -INFINITY : 0.f, l = 0.f;
     bool ok = true;
     int ks_slot = 0;

@@ -89,9 +89,10 @@ def per_block_int8(q: torch.Tensor, k: torch.Tensor, km: Optional[torch.Tensor] 
 
 
 def quantize_operands(qb: torch.Tensor, kb: torch.Tensor, sm_scale: float, smooth_k: bool,
-                      scale_granularity: Optional[str] = None):
+                      scale_granularity: Optional[str] = None, alias_q: bool = False):
     """Operand preparation (``hq_prefill_quant`` / ``hq_prefill_quant_blocks``): returns q_i8, q_bf, q_scale, k_i8,
-    k_bf, k_scale, k_mean; the scale arrays hold one value per row either way."""
+    k_bf, k_scale, k_mean; the scale arrays hold one value per row either way.  ``alias_q``: q_bf may be ``qb`` itself
+    (the BF16 query operand is the query row by row, so a contiguous query needs no copy)."""
     gran = SCALE_GRANULARITY if scale_granularity is None else scale_granularity
     if gran not in ("row", "block"):
         raise ValueError(f"scale_granularity must be 'row' or 'block', got {gran!r}")
@@ -101,11 +102,13 @@ def quantize_operands(qb: torch.Tensor, kb: torch.Tensor, sm_scale: float, smoot
     lib = _lib.lib()
     nqb, nkb = (N + 127) // 128, (N + 63) // 64
     q_i8 = torch.empty(B, H_q, N, 128, dtype=torch.int8, device=dev)
-    q_bf = torch.empty(B, H_q, N, 128, dtype=torch.bfloat16, device=dev)
-    q_sc = torch.zeros(B, H_q, (N + 63) // 64 * 64, dtype=torch.float32, device=dev)
+    alias_q = alias_q and gran == "row" and qb.is_contiguous()
+    q_bf = qb if alias_q else torch.empty(B, H_q, N, 128, dtype=torch.bfloat16, device=dev)
+    scales = torch.empty if gran == "row" else torch.zeros         # the row quantiser writes the padding rows itself
+    q_sc = scales(B, H_q, (N + 63) // 64 * 64, dtype=torch.float32, device=dev)
     k_i8 = torch.empty(B, H_kv, N, 128, dtype=torch.int8, device=dev)
     k_bf = torch.empty(B, H_kv, N, 128, dtype=torch.bfloat16, device=dev)
-    k_sc = torch.zeros(B, H_kv, (N + 63) // 64 * 64, dtype=torch.float32, device=dev)
+    k_sc = scales(B, H_kv, (N + 63) // 64 * 64, dtype=torch.float32, device=dev)
     k_mean = torch.empty(B, H_kv, 128, dtype=torch.bfloat16, device=dev)
     nb = C.c_int64(0)
     _lib.check(lib.hq_prefill_quant_workspace_bytes(B, H_kv, C.byref(nb)), "hq_prefill_quant_workspace_bytes")
@@ -127,9 +130,11 @@ class PrefillPlan:
 
     def __init__(self, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, vertical_indices: Optional[torch.Tensor],
                  window_size: int, sm_scale: Optional[float], smooth_k: bool, scale_granularity: Optional[str] = None,
-                 pv_fp8: bool = False):
-        """``pv_fp8``: the P V product in FP8 E4M3 with the reference's ``sage_fp8_attention`` arithmetic (V^T quantised
-        per channel, P~ = 2^(s - m + 8.807) against the exact running maximum), for INT8, window and vertical tiles alike."""
+                 pv_fp8: bool = False, alias_inputs: bool = False):
+        """``alias_inputs``: the caller runs the plan before it changes q, k or v, so that operands which are equal to
+        an input may be that input.  ``pv_fp8``: the P V product in FP8 E4M3 with the reference's ``sage_fp8_attention``
+        arithmetic (V^T quantised per channel, P~ = 2^(s - m + 8.807) against the exact running maximum), for INT8,
+        window and vertical tiles alike."""
         dtype = q.dtype
         qb, kb, vb, B, H_q, H_kv, N = _prep_inputs(q, k, v)
         dev = q.device
@@ -138,7 +143,16 @@ class PrefillPlan:
         if sm_scale is None:
             sm_scale = 128 ** -0.5
         nqb, nkb = (N + 127) // 128, (N + 63) // 64
-        q_i8, q_bf, q_sc, k_i8, k_bf, k_sc, k_mean = quantize_operands(qb, kb, sm_scale, smooth_k, scale_granularity)
+        # A window that covers the prompt leaves no INT8 tile and no vertical line (16-bit causal attention): without K
+        # smoothing the BF16 operands are then q and k as they are, and nothing reads codes, scales or biases
+        # (2 x 32 heads x 1973 tokens: 54 of 189 us were spent on them).
+        bf16_only = alias_inputs and window_size >= N and not smooth_k and N > 0
+        if bf16_only:
+            q_bf, k_bf = qb.contiguous(), kb.contiguous()
+            q_i8 = q_sc = q_bf
+            k_i8 = k_sc = k_mean = k_bf
+        else:
+            q_i8, q_bf, q_sc, k_i8, k_bf, k_sc, k_mean = quantize_operands(qb, kb, sm_scale, smooth_k, scale_granularity, alias_inputs)
         T = 0
         vert_k = vert_vt = nvv = vasc = None
         Npad = (N + 63) // 64 * 64
@@ -157,17 +171,23 @@ class PrefillPlan:
         if vertical_indices is not None and vertical_indices.shape[-1] > 0 and prefix_len > 0:
             if tuple(vertical_indices.shape[:2]) != (B, H_q):
                 raise HyQuantError("vertical_indices must be [B, H_q, T]")
-            vid = vertical_indices.to(device=dev, dtype=torch.int64).clamp(0, prefix_len - 1)   # reference :510
-            vasc = vid.sort(dim=-1).values.to(torch.int32).contiguous()
-            T = int(vasc.shape[-1])
+            vid = vertical_indices.to(device=dev, dtype=torch.int64)
+            T = int(vid.shape[-1])
+            if T <= 16384 and prefix_len <= 1 << 20:
+                vid = vid.contiguous()
+                vasc = torch.empty(B, H_q, T, dtype=torch.int32, device=dev)
+                _lib.check(lib.hq_prefill_vertical_sort(vid.data_ptr(), B * H_q, T, prefix_len - 1, vasc.data_ptr(), st),
+                           "hq_prefill_vertical_sort")
+            else:
+                vasc = vid.clamp(0, prefix_len - 1).sort(dim=-1).values.to(torch.int32).contiguous()   # reference :510
             Tpad = (T + 63) // 64 * 64
             vert_k = torch.empty(B, H_q, Tpad, 128, dtype=torch.bfloat16, device=dev)
             vert_vt = torch.empty(B, H_q, 128, Tpad, dtype=torch.bfloat16, device=dev)
             nvv = torch.empty(B, H_q, nqb, dtype=torch.int32, device=dev)
         # per (query head, key) term of the INT8 score conversion; -inf on the head's vertical lines
-        k_bias = torch.empty(B, H_q, Npad, dtype=torch.float32, device=dev)
         ptr = lambda t: None if t is None else t.data_ptr()     # noqa: E731
-        rc = lib.hq_prefill_vertical_prepare(ptr(vasc), B, H_q, H_kv, N, window_size, T, k_bf.data_ptr(),
+        k_bias = k_bf if bf16_only else torch.empty(B, H_q, Npad, dtype=torch.float32, device=dev)
+        rc = 0 if bf16_only else lib.hq_prefill_vertical_prepare(ptr(vasc), B, H_q, H_kv, N, window_size, T, k_bf.data_ptr(),
                                              vb.data_ptr(), vb.stride(0), vb.stride(1), vb.stride(2), k_sc.data_ptr(),
                                              ptr(vert_k), ptr(vert_vt), k_bias.data_ptr(), ptr(nvv), st)
         _lib.check(rc, "hq_prefill_vertical_prepare")
@@ -218,7 +238,7 @@ def hybrid_prefill(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, vertical_i
                    scale_granularity: Optional[str] = None, pv_fp8: bool = False) -> torch.Tensor:
     """Causal attention [B,H_q,N,D] with INT8 QK^T on the non-vertical prefix and BF16 on the
     vertical lines and the window.  ``vertical_indices`` int64 [B,H_q,T] (any order) or None."""
-    return PrefillPlan(q, k, v, vertical_indices, window_size, sm_scale, smooth_k, scale_granularity, pv_fp8).run()
+    return PrefillPlan(q, k, v, vertical_indices, window_size, sm_scale, smooth_k, scale_granularity, pv_fp8, alias_inputs=True).run()
 
 
 def sage_vertical_attention_v2(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, vertical_indices: torch.Tensor, *,

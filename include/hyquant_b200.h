@@ -322,7 +322,7 @@ int hq_cache_reorganize_bits(const void* keys, const void* values, int64_t kv_st
  * (src/ops/vendor/sageattention/triton/quant_per_block.py:21-101,
  *  src/ops/sage_unified.py:565-576).
  *   q [B,H_Q,N,128] bf16, k [B,H_KV,N,128] bf16 (strides in elements)
- *   q_i8 int8 [B,H_Q,N,128], q_bf bf16 (contiguous copy of q), q_scale fp32 [B,H_Q,Npad] (one per row; Npad = N rounded up to 64)
+ *   q_i8 int8 [B,H_Q,N,128], q_bf bf16 (contiguous copy of q; may be q itself if q is contiguous), q_scale fp32 [B,H_Q,Npad] (one per row; Npad = N rounded up to 64)
  *   k_i8 int8 [B,H_KV,N,128], k_bf bf16 (k - mean), k_scale fp32 [B,H_KV,Npad], k_mean bf16 [B,H_KV,128]
  * smooth_k == 0 leaves K unshifted.
  */
@@ -355,6 +355,11 @@ int hq_prefill_quant_blocks(const void* q, int64_t q_sb, int64_t q_sh, int64_t q
 int hq_per_block_int8(const void* x, int64_t x_sb, int64_t x_sh, int64_t x_sn, int B, int H, int L, int blk,
                       float mul, const void* mean, void* x_i8, int64_t o_sb, int64_t o_sh, int64_t o_sn,
                       float* scale, void* stream);
+
+/* The index lists hq_prefill_vertical_prepare wants: vidx int64 [rows, T] in any order (as hq_topk and torch.topk give
+ * them) -> vidx_asc int32 [rows, T], clamped to [0, last] (reference src/ops/sage_unified.py:510) and ascending; a position
+ * given twice stays twice.  T up to 16384, last below 2^20. */
+int hq_prefill_vertical_sort(const int64_t* vidx, int rows, int T, int last, int32_t* vidx_asc, void* stream);
 
 /* Step 2: vertical-line bookkeeping.  Replaces reorder_kv_for_vertical
  * (src/ops/sage_unified.py:499-547) without expanding K/V to query heads:

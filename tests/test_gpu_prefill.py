@@ -56,6 +56,52 @@ def test_operand_preparation_bit_exact(N, smooth):
     assert np.array_equal(to_np(q_bf), q)
 
 
+def test_row_codes_on_and_beside_ties():
+    """Rows whose quotients are half-integers or one step beside them, all-zero rows, rows of the smallest values: the
+    codes of the division, bit for bit (the kernel multiplies by the reciprocal except near a tie)."""
+    rng = np.random.Generator(np.random.PCG64(3))
+    N = 333
+    k = (rng.integers(-127, 127, size=(1, 2, N, 128)) + 0.5).astype(np.float32)
+    k[:, :, :, 0] = 127.0                                    # scale 2^e: every quotient is a half-integer
+    k *= (2.0 ** rng.integers(-12, 12, size=(1, 2, N, 1))).astype(np.float32)
+    k[:, :, 100:200] = orc.bf16_round(k[:, :, 100:200] * np.float32(1.0078125))       # beside the ties
+    k[:, :, 200:220] *= rng.uniform(0.5, 2.0, size=(1, 2, 20, 1)).astype(np.float32)
+    k[:, :, 220] = 0.0
+    k[:, :, 221] = 1e-38
+    k = orc.bf16_round(k)
+    q = orc.bf16_round(rng.standard_normal((1, 4, N, 128), dtype=np.float32))
+    _, _, _, k_i8, _, k_sc, _ = su.quantize_operands(t_bf16(q), t_bf16(k), 128 ** -0.5, False)
+    ki, ks = orc.quant_per_block_int8(k, 1, 1.0)
+    live = np.ones(N, bool); live[220:222] = False           # the oracle divides a zero row by zero
+    assert np.array_equal(k_i8.cpu().numpy()[:, :, live], ki[:, :, live])
+    assert np.array_equal(k_sc.cpu().numpy()[..., :N][..., live], ks[..., live])
+    assert not k_i8.cpu().numpy()[:, :, 220:222].any()
+
+
+@pytest.mark.parametrize("T,last", [(1, 0), (64, 63), (65, 4000), (1600, 32639), (500, 100), (16384, (1 << 20) - 1)])
+def test_vertical_sort_is_the_clamped_ascending_list(T, last):
+    """Positions out of range and positions given twice (or T times) among them."""
+    g = torch.Generator(device=DEV); g.manual_seed(T)
+    idx = torch.randint(-3, last + 5, (3, T), generator=g, device=DEV)
+    if T <= 1600:
+        idx[1] = last // 2
+    asc = torch.empty(3, T, dtype=torch.int32, device=DEV)
+    lib = hq._lib.lib()
+    assert lib.hq_prefill_vertical_sort(idx.data_ptr(), 3, T, last, asc.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+    assert torch.equal(asc.long(), idx.clamp(0, last).sort(dim=-1).values)
+
+
+def test_the_one_shot_calls_leave_their_inputs_alone():
+    """The one-shot entry points may read q and k in place where a plan copies them: same result, inputs unchanged."""
+    q, k, v = make(2, 4, 2, 333, 128, 3)
+    for window, smooth in ((128, True), (333, False), (500, False), (0, True)):
+        tq, tk, tv = t_bf16(q), t_bf16(k), t_bf16(v)
+        a = su.hybrid_prefill(tq, tk, tv, None, window, None, smooth)
+        b = su.PrefillPlan(tq, tk, tv, None, window, None, smooth).run()
+        assert torch.equal(a, b)
+        assert np.array_equal(to_np(tq), q) and np.array_equal(to_np(tk), k) and np.array_equal(to_np(tv), v)
+
+
 def check(out, ref):
     assert np.isfinite(out).all()
     assert max_abs(out, ref) <= MAX_ABS, max_abs(out, ref)

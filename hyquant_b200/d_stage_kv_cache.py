@@ -378,10 +378,12 @@ class DStageLayerCache:
         return self._staging_ptr >= GROUP_SIZE - 1
 
     def capture_decode_step(self, query_states, key_states, value_states, kv_repeat: int, out: torch.Tensor,
-                            overlap: bool = True):
+                            overlap: bool = True, num_splits: int = 0, workspace: Optional[torch.Tensor] = None):
         """Issue the fused ``decode_step`` launch WITHOUT counting the token: for use inside a CUDA-graph capture
         (lengths bound with :meth:`bind_lengths`; every tensor argument must keep its address across replays).
-        After each replay call :meth:`count_replayed_step`."""
+        After each replay call :meth:`count_replayed_step`.  ``num_splits`` (0 = chosen for this launch alone) and
+        ``workspace`` (split-K scratch, ``hq_decode_workspace_bytes``, zero-filled; kept by the caller): for launches
+        that share the chip with others on other branches of the graph."""
         if self._lengths is None:
             raise HyQuantError("bind_lengths first: a captured launch must not carry the lengths in its arguments")
         B, H_KV, S, D = key_states.shape
@@ -390,12 +392,17 @@ class DStageLayerCache:
         k2, v2 = key_states.reshape(B * H_KV, D), value_states.reshape(B * H_KV, D)
         plan = self._decode_plan(q2d, kv_repeat)
         a = plan.args
+        own = (a.num_splits, a.workspace, a.workspace_bytes, a.flags)
         a.flags = _lib.HQ_DECODE_OVERLAP_PREVIOUS if (overlap and self.k_bits == 4 and self.v_bits == 4) else 0
         a.k_new, a.v_new, a.kn_stride, a.vn_stride = k2.data_ptr(), v2.data_ptr(), k2.stride(0), v2.stride(0)
+        a.num_splits = num_splits
+        if workspace is not None:
+            a.workspace, a.workspace_bytes = workspace.data_ptr(), workspace.numel()
         try:
             plan.run(q2d, out=out.view(B_ * H_Q_, D_))
         finally:
             a.k_new = a.v_new = None
+            a.num_splits, a.workspace, a.workspace_bytes, a.flags = own
 
     def count_replayed_step(self):
         """Account for one replay of a launch captured by :meth:`capture_decode_step` (one token appended)."""

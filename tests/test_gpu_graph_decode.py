@@ -62,6 +62,29 @@ def test_graph_replay_equals_layer_by_layer_across_flushes():
     assert torch.equal(layers[0].decode_attention(q, R), ref_layers[0].decode_attention(q, R))
 
 
+@pytest.mark.parametrize("n,B,H_Q,H_KV,N,W", [(1, 1, 4, 2, 300, 64), (2, 1, 8, 8, 200, 64), (11, 1, 4, 2, 700, 64), (17, 2, 16, 1, 450, 128)])
+def test_layers_on_branches_equal_layer_by_layer(n, B, H_Q, H_KV, N, W):
+    """One layer, fewer layers than branches, more layers than branches, sixteen query heads per kv-head (another split
+    count each): every replay against the layer-by-layer path, and the rows each layer staged."""
+    R = H_Q // H_KV
+    ref_layers, layers = _layers(n, B, H_Q, H_KV, N, W), _layers(n, B, H_Q, H_KV, N, W)
+    g = DecodeStepGraph(layers, B, H_Q, H_KV)
+    gen = torch.Generator(); gen.manual_seed(n)
+    for s in range(6):
+        rows = torch.randn(n, B, H_Q + 2 * H_KV, 1, 128, generator=gen).to(torch.bfloat16)
+        q, k, v = rows[:, :, :H_Q], rows[:, :, H_Q:H_Q + H_KV], rows[:, :, H_Q + H_KV:]
+        for i in range(n):
+            g.host_q[i].copy_(q[i]); g.host_k[i].copy_(k[i]); g.host_v[i].copy_(v[i])
+        out = g.step().clone()
+        for i in range(n):
+            ref = ref_layers[i].decode_step(q[i].to(DEV), k[i].to(DEV), v[i].to(DEV), R)
+            assert (out[i].to(DEV).float() - ref.float()).abs().max().item() <= 2e-3, (s, i)
+    for i in range(n):
+        assert torch.equal(layers[i]._staging_buf_k, ref_layers[i]._staging_buf_k)
+        assert torch.equal(layers[i]._staging_buf_v, ref_layers[i]._staging_buf_v)
+    g.close()
+
+
 def test_lengths_record_overrides_the_arguments():
     """The kernel must follow the device record, not the launch arguments."""
     (layer,) = _layers(1, 1, 8, 2, 900, 64)

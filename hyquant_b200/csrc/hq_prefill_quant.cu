@@ -59,17 +59,33 @@ __global__ void kmean_final_kernel(const float* __restrict__ partial, int N, int
 // One INT8 scale per ROW (token): scale = max|x| / 127, code = x / scale rounded half away from zero; rows N ..
 // scale_pitch - 1 get scale 0.
 //
-// Eight lanes per row, sixteen channels each, 32 rows per CTA.  Sixteen IEEE divisions a lane were what the kernel waited
-// for: the product with the rounded reciprocal is within 1.5 * 2^-23 of the quotient, relatively, and |quotient| <= 127
-// (1 + 2^-22), so it rounds to the same integer unless it lies within kNearTie of a half-integer; only then the
-// division is done.  Infinite and NaN inputs as the division gives them: x / inf = x * 0, inf / inf = inf * 0 = NaN,
-// which the clamp turns into the lowest code.  Queries of 32 heads x 8192 rows with their copy: 49 us before.
+// Eight lanes per row, sixteen channels each, 32 rows per CTA.  Bound by instruction issue before HBM, so the work per
+// element is kept small: the row maximum on pairs of bf16 bit patterns, everything else on magnitudes, two to an
+// instruction, the sign put back on four packed bytes at a time.  Rounding half away from zero is |y| + 0.5 cut off, and
+// y has to be the correctly rounded quotient (a bf16 value over a 127th of another lies exactly on a tie often enough
+// that falling back near ties meant falling back in most warps): Markstein's division (IBM J. Res. Dev. 34, 1990),
+// the product with the rounded reciprocal corrected once by its exact remainder.  Rows whose maximum is infinite, NaN or
+// out of that method's range take the divide instruction element by element: x / inf = 0, inf / inf = NaN, which the
+// clamp turns into the lowest code.
+__device__ __noinline__ void row_codes_exact(const float (&v)[16], float sc, uint32_t (&code)[4]) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    uint32_t c = 0;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      float y = __fdiv_rn(v[4 * i + e], sc);
+      y += y >= 0.f ? 0.5f : -0.5f;
+      c |= ((uint32_t)(int)fminf(fmaxf(truncf(y), -128.f), 127.f) & 0xFFu) << (8 * e);
+    }
+    code[i] = c;
+  }
+}
+
 template <bool kIsK>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 5)
 row_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t sb, int64_t sh, int64_t sn, int H, int N,
                  const __nv_bfloat16* __restrict__ mean, float mul,
                  int8_t* __restrict__ xi8, __nv_bfloat16* __restrict__ xbf, float* __restrict__ scale, int scale_pitch) {
-  constexpr float kNearTie = 1.5e-4f;
   const int bh = blockIdx.y, b = bh / H, h = bh - b * H;
   const int tid = threadIdx.x;
   const int row = blockIdx.x * 32 + (tid >> 3), c = (tid & 7) * 16;
@@ -80,10 +96,8 @@ row_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t sb, int64_t sh, in
     raw[0] = __ldg(src); raw[1] = __ldg(src + 1);
   }
   uint32_t w[8] = {raw[0].x, raw[0].y, raw[0].z, raw[0].w, raw[1].x, raw[1].y, raw[1].z, raw[1].w};
-  float v[16];
-  float amax = 0.f;
-  uint32_t mw[8];
   if (kIsK) {
+    uint32_t mw[8];
     const __nv_bfloat16* mp = mean + (int64_t)bh * 128 + c;
     if ((reinterpret_cast<uintptr_t>(mp) & 15) == 0) {
       const uint4 m0 = __ldg(reinterpret_cast<const uint4*>(mp)), m1 = __ldg(reinterpret_cast<const uint4*>(mp) + 1);
@@ -93,22 +107,20 @@ row_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t sb, int64_t sh, in
 #pragma unroll
       for (int j = 0; j < 8; ++j) mw[j] = (uint32_t)__ldg(e + 2 * j) | ((uint32_t)__ldg(e + 2 * j + 1) << 16);
     }
-  }
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    float f0 = __uint_as_float(w[j] << 16), f1 = __uint_as_float(w[j] & 0xFFFF0000u);
-    if (kIsK) {
-      const __nv_bfloat162 d = __floats2bfloat162_rn(f0 - __uint_as_float(mw[j] << 16), f1 - __uint_as_float(mw[j] & 0xFFFF0000u));
+    for (int j = 0; j < 8; ++j) {
+      const __nv_bfloat162 d = __floats2bfloat162_rn(__uint_as_float(w[j] << 16) - __uint_as_float(mw[j] << 16),
+                                                     __uint_as_float(w[j] & 0xFFFF0000u) - __uint_as_float(mw[j] & 0xFFFF0000u));
       w[j] = *reinterpret_cast<const uint32_t*>(&d);
-      f0 = __uint_as_float(w[j] << 16); f1 = __uint_as_float(w[j] & 0xFFFF0000u);
-    } else {
-      f0 *= mul; f1 *= mul;
     }
-    v[2 * j] = f0; v[2 * j + 1] = f1;
-    amax = fmaxf(amax, fmaxf(fabsf(f0), fabsf(f1)));
   }
+  // max|x| over the row: magnitudes of bf16 values order like their bit patterns, NaN above infinity
+  uint32_t pm = 0u;
 #pragma unroll
-  for (int o = 4; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+  for (int j = 0; j < 8; ++j) pm = __vmaxu2(pm, w[j] & 0x7FFF7FFFu);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) pm = __vmaxu2(pm, __shfl_xor_sync(0xffffffffu, pm, o));
+  const uint32_t top = max(pm & 0xFFFFu, pm >> 16);
   if (!ok) {
     if ((tid & 7) == 0 && row < scale_pitch) scale[(int64_t)bh * scale_pitch + row] = 0.f;
     return;
@@ -118,35 +130,51 @@ row_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t sb, int64_t sh, in
     dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
     dst[1] = make_uint4(w[4], w[5], w[6], w[7]);
   }
-  const float sc = fmaxf(amax, 1e-30f) / 127.f;     // an all-zero row keeps codes 0 instead of NaN
+  float amax = __uint_as_float(top << 16) * (kIsK ? 1.0f : fabsf(mul));
+  if (top > 0x7F80u) {                                  // a NaN in the row does not count for its maximum
+    amax = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      amax = fmaxf(amax, fmaxf(fabsf(__uint_as_float(w[j] << 16) * (kIsK ? 1.0f : mul)), fabsf(__uint_as_float(w[j] & 0xFFFF0000u) * (kIsK ? 1.0f : mul))));
+    const uint32_t lanes = 0xFFu << (tid & 24);         // the row's eight lanes are here together
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(lanes, amax, o));
+  }
+  const float sc = __fdiv_rn(fmaxf(amax, 1e-30f), 127.f);     // an all-zero row keeps codes 0 instead of NaN
   if ((tid & 7) == 0) scale[(int64_t)bh * scale_pitch + row] = sc;
   const float rcp = __frcp_rn(sc);
-  float far = 0.f;
+  const float2 rcp2 = make_float2(rcp, rcp), nsc2 = make_float2(-sc, -sc), half2 = make_float2(0.5f, 0.5f);
+  const float2 big2 = make_float2(8388608.f, 8388608.f), mul2 = make_float2(fabsf(mul), fabsf(mul));
+  const uint32_t turn = !kIsK && mul < 0.f ? 0xFFFFFFFFu : 0u;
+  // two magnitudes of a word -> floor(quotient + 0.5) in the low mantissa bits
+  auto two = [&](uint32_t word) -> float2 {
+    const uint32_t m = word & 0x7FFF7FFFu;
+    float2 v = make_float2(__uint_as_float(m << 16), __uint_as_float(m & 0xFFFF0000u));
+    if (!kIsK) v = fmul2(v, mul2);
+    const float2 q = fmul2(v, rcp2);
+    const float2 y = ffma2(ffma2(q, nsc2, v), rcp2, q);
+    return fadd2_rz(fadd2(y, half2), big2);
+  };
   uint32_t code[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    uint32_t r[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float t = fminf(fmaxf(__fmul_rn(v[4 * i + e], rcp), -128.f), 127.f);
-      const float y = __fadd_rn(t, 12582912.f);              // rounds to an integer, which the low mantissa bits then hold
-      far = fmaxf(far, fabsf(__fsub_rn(t, __fsub_rn(y, 12582912.f))));
-      r[e] = __float_as_uint(y);
-    }
-    code[i] = prmt(prmt(r[0], r[1], 0x0040), prmt(r[2], r[3], 0x0040), 0x5410);
+    const float2 r0 = two(w[2 * i]), r1 = two(w[2 * i + 1]);
+    const uint32_t n = prmt(prmt(__float_as_uint(r0.x), __float_as_uint(r0.y), 0x0040), prmt(__float_as_uint(r1.x), __float_as_uint(r1.y), 0x0040), 0x5410);
+    const uint32_t neg = prmt(w[2 * i], w[2 * i + 1], 0xFDB9) ^ turn;       // 0xFF in the bytes of negative elements
+    const uint32_t flipped = n ^ neg;                                       // n <= 127: minus n is its complement plus one
+    code[i] = ((flipped & 0x7F7F7F7Fu) + (neg & 0x01010101u)) ^ (flipped & 0x80808080u);
   }
-  if (far > 0.5f - kNearTie) {
+  if (!(amax >= 1e-25f && amax <= 1e30f)) {
+    float v[16];                        // arrays of their own: what goes to the call by address must not be the common path's
+    uint32_t exact[4];
 #pragma unroll
-    for (int e = 0; e < 16; ++e) {
-      const float t = __fmul_rn(v[e], rcp);
-      if (0.5f - fabsf(t - rintf(t)) < kNearTie) {
-        float y = __fdiv_rn(v[e], sc);
-        y += y >= 0.f ? 0.5f : -0.5f;
-        const int q = (int)fminf(fmaxf(truncf(y), -128.f), 127.f);
-        const uint32_t m = 0xFFu << (8 * (e & 3));
-        code[e >> 2] = (code[e >> 2] & ~m) | (((uint32_t)q << (8 * (e & 3))) & m);
-      }
+    for (int j = 0; j < 8; ++j) {
+      v[2 * j] = __uint_as_float(w[j] << 16); v[2 * j + 1] = __uint_as_float(w[j] & 0xFFFF0000u);
+      if (!kIsK) { v[2 * j] *= mul; v[2 * j + 1] *= mul; }
     }
+    row_codes_exact(v, sc, exact);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) code[j] = exact[j];
   }
   int8_t* out = xi8 + ((int64_t)bh * N + row) * 128 + c;       // 8-byte aligned at least
   if ((reinterpret_cast<uintptr_t>(out) & 15) == 0) {

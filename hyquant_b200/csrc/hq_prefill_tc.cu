@@ -56,21 +56,6 @@ struct TcSmem {              // offsets from a 1024-aligned base
   static constexpr int Total = Bar + 256;
 };
 
-// two fp32 lanes per instruction (sm_100 packed forms)
-__device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
-  float2 d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(*reinterpret_cast<unsigned long long*>(&d))
-      : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)),
-        "l"(*reinterpret_cast<unsigned long long*>(&c)));
-  return d;
-}
-__device__ __forceinline__ float2 fadd2(float2 a, float2 b) {
-  float2 d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(*reinterpret_cast<unsigned long long*>(&d))
-      : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)));
-  return d;
-}
-
 struct TcPlan {
   int n_rest, n_win, nvert0, nvert1, nheads;
   __device__ __forceinline__ int nvert(int h) const { return h ? nvert1 : nvert0; }

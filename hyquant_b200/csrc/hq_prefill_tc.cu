@@ -107,7 +107,28 @@ struct TcSlowResult { float m_ref, l; bool ok; };
 // qk_int_sv_f8_cuda_sm90.cu:259-364): P~ = 2^(s - m + 8.807) against the EXACT running maximum m (so P~ <= 448, the largest
 // e4m3 value), the row sum taken in fp32 before P~ is rounded to e4m3.
 constexpr float kFp8Offset = 8.807f;
-template <bool kFp8>
+
+// compile-time flag handed to a lambda
+struct TcTrue { static constexpr bool value = true; };
+struct TcFalse { static constexpr bool value = false; };
+
+// O of a row times alpha, in tensor memory, once every P V issued so far has completed.  Whole warps.
+__device__ __noinline__ bool tc_rescale_o(uint32_t tO, float alpha, uint64_t* pv_bar, uint32_t pv_parity, volatile int* abort_flag) {
+  if (!__all_sync(0xffffffffu, tc::mbar_wait_abortable(pv_bar, pv_parity, abort_flag))) return false;
+  tc::fence_after_sync();
+#pragma unroll
+  for (int ch = 0; ch < 4; ++ch) {
+    uint32_t o[32];
+    tc::tmem_ld32(tO + ch * 32, o);
+    tc::tmem_wait_ld();
+#pragma unroll
+    for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * alpha);
+    tc::tmem_st32(tO + ch * 32, o);
+  }
+  tc::tmem_wait_st();
+  return true;
+}
+
 __device__ __noinline__ TcSlowResult tc_slow_tile(uint32_t tS, uint32_t tO, const float4* ks4, const float4* kb4, bool is_i8,
                                                   float esc, uint32_t mlo, uint32_t mhi, float m_ref, float l,
                                                   uint64_t* pv_bar, uint32_t pv_parity, volatile int* abort_flag) {
@@ -144,46 +165,22 @@ __device__ __noinline__ TcSlowResult tc_slow_tile(uint32_t tS, uint32_t tO, cons
   if (__any_sync(0xffffffffu, grow)) {
     const float alpha = (m_ref == -INFINITY) ? 0.f : ex2f(m_ref - mx);
     if (pv_bar != nullptr) {   // O must be quiescent: every P V of this head issued so far has to be complete
-      res.ok = __all_sync(0xffffffffu, tc::mbar_wait_abortable(pv_bar, pv_parity, abort_flag));
+      res.ok = tc_rescale_o(tO, grow ? alpha : 1.f, pv_bar, pv_parity, abort_flag);
       if (!res.ok) { res.m_ref = m_ref; res.l = l; return res; }
-      tc::fence_after_sync();
-#pragma unroll
-      for (int ch = 0; ch < 4; ++ch) {
-        uint32_t o[32];
-        tc::tmem_ld32(tO + ch * 32, o);
-        tc::tmem_wait_ld();
-#pragma unroll
-        for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * (grow ? alpha : 1.f));
-        tc::tmem_st32(tO + ch * 32, o);
-      }
-      tc::tmem_wait_st();
     }
     if (grow) { l *= alpha; m_ref = mx; }
   }
   const float mu = m_ref == -INFINITY ? 0.f : m_ref;
   float rs[4] = {0.f, 0.f, 0.f, 0.f};
-  if constexpr (kFp8) {
-    uint32_t pk[16];
-    const float off = kFp8Offset - mu;
+  uint32_t pk[32];
 #pragma unroll
-    for (int c = 0; c < 64; c += 4) {
-      const float p0 = ex2f(fmaf(x[c], esc, off)), p1 = ex2f(fmaf(x[c + 1], esc, off));
-      const float p2 = ex2f(fmaf(x[c + 2], esc, off)), p3 = ex2f(fmaf(x[c + 3], esc, off));
-      rs[0] += p0; rs[1] += p1; rs[2] += p2; rs[3] += p3;
-      pk[c >> 2] = tc::pack_e4m3x4(p0, p1, p2, p3);
-    }
-    tc::tmem_st16(tS, pk);
-  } else {
-    uint32_t pk[32];
-#pragma unroll
-    for (int c = 0; c < 64; c += 2) {
-      const float p0 = ex2f(fmaf(x[c], esc, -mu)), p1 = ex2f(fmaf(x[c + 1], esc, -mu));
-      rs[c & 3] += p0; rs[(c & 3) + 1] += p1;
-      __nv_bfloat162 hh = __floats2bfloat162_rn(p0, p1);       // low half = even column
-      pk[c >> 1] = *reinterpret_cast<uint32_t*>(&hh);
-    }
-    tc::tmem_st32(tS, pk);
+  for (int c = 0; c < 64; c += 2) {
+    const float p0 = ex2f(fmaf(x[c], esc, -mu)), p1 = ex2f(fmaf(x[c + 1], esc, -mu));
+    rs[c & 3] += p0; rs[(c & 3) + 1] += p1;
+    __nv_bfloat162 hh = __floats2bfloat162_rn(p0, p1);       // low half = even column
+    pk[c >> 1] = *reinterpret_cast<uint32_t*>(&hh);
   }
+  tc::tmem_st32(tS, pk);
   tc::tmem_wait_st();
   res.m_ref = m_ref;
   res.l = l + (rs[0] + rs[1]) + (rs[2] + rs[3]);
@@ -335,41 +332,51 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap mQi, const __grid_constant
       cq.begin(plan, kKStages);
       cp.begin(plan, kVStages);
       int tq = 0;
-      auto qk_next = [&]() {
-        for (;;) {          // the next item that feeds this head; hand back the other head's on the way
+      auto k_ready = [&]() {     // wait for the next item that feeds this head; hand back the other head's on the way
+        for (;;) {
           ok = wait(k_full + cq.stage, cq.par);
-          if (!ok) return;
-          if (cq.feeds(h)) break;
+          if (!ok || cq.feeds(h)) return;
           if (tc::elect_one()) tc::mbar_arrive(k_empty + cq.stage);
           cq.next(plan);
         }
-        tc::fence_after_sync();
-        const uint32_t dS = tS + 64u * (tq & 1);
-        const uint64_t bK = dK + (uint64_t)(cq.stage * 1024);
-        if (tc::elect_one()) {
-          if (cq.kind == 0) {
-#pragma unroll
-            for (int k = 0; k < 4; ++k) tc::mma_s8_ss(dS, dQi + 2 * k, bK + 2 * k, idesc_i8, k > 0);
-          } else {
-#pragma unroll
-            for (int k = 0; k < 8; ++k)
-              tc::mma_bf16_ss(dS, dQb + (k >> 2) * 1024 + 2 * (k & 3), bK + (k >> 2) * 512 + 2 * (k & 3), idesc_qk, k > 0);
-          }
-          tc::mma_commit(s_full + 2 * h + (tq & 1));
-          tc::mma_commit(k_empty + cq.stage);
-        }
-        ++tq;
-        cq.next(plan);
       };
-      if (ok && n_t > 0) qk_next();
-      if (ok && n_t > 1) qk_next();
-      for (int t = 0; ok && t < n_t; ++t) {
+      auto v_ready = [&]() {
         for (;;) {
           ok = wait(v_full + cp.stage, cp.par);
-          if (!ok || cp.feeds(h)) break;
+          if (!ok || cp.feeds(h)) return;
           if (tc::elect_one()) tc::mbar_arrive(v_empty + cp.stage);
           cp.next(plan);
         }
+      };
+      auto qk_issue = [&]() {    // one lane
+        const uint32_t dS = tS + 64u * (tq & 1);
+        const uint64_t bK = dK + (uint64_t)(cq.stage * 1024);
+        if (cq.kind == 0) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) tc::mma_s8_ss(dS, dQi + 2 * k, bK + 2 * k, idesc_i8, k > 0);
+        } else {
+#pragma unroll
+          for (int k = 0; k < 8; ++k)
+            tc::mma_bf16_ss(dS, dQb + (k >> 2) * 1024 + 2 * (k & 3), bK + (k >> 2) * 512 + 2 * (k & 3), idesc_qk, k > 0);
+        }
+        tc::mma_commit(s_full + 2 * h + (tq & 1));
+        tc::mma_commit(k_empty + cq.stage);
+      };
+      for (int i = 0; i < 2 && i < n_t; ++i) {
+        if (ok) k_ready();
+        if (!ok) break;
+        tc::fence_after_sync();
+        if (tc::elect_one()) qk_issue();
+        ++tq;
+        cq.next(plan);
+      }
+      for (int t = 0; ok && t < n_t; ++t) {
+        // the operands first, P last: from the moment P is there nothing is waited for, and P V of t and Q K^T of t + 2
+        // are issued together (a wait costs the warp some 400 clocks even if what it waits for is there: 32K hybrid
+        // 9.27 -> 9.05 ms, 8K 867 -> 844 us)
+        const bool more = t + 2 < n_t;
+        v_ready();
+        if (ok && more) k_ready();
         if (!ok) break;
         const int sl = 2 * h + (t & 1);
         ok = wait(p_ready + sl, (uint32_t)((t >> 1) & 1));
@@ -387,9 +394,10 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap mQi, const __grid_constant
           }
           tc::mma_commit(pv_done + sl);
           tc::mma_commit(v_empty + cp.stage);
+          if (more) qk_issue();
         }
         cp.next(plan);
-        if (t + 2 < n_t) qk_next();
+        if (more) { ++tq; cq.next(plan); }
       }
     }
   } else {
@@ -408,89 +416,131 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap mQi, const __grid_constant
     float m_ref = row < p.N ? -INFINITY : 0.f, l = 0.f;
     bool ok = true;
     int ks_slot = 0;
-    for (int t = 0; t < n_tiles; ++t) {
-      const int slot = t & 1, sl = 2 * h + slot;
-      ok = __all_sync(0xffffffffu, tc::mbar_wait_abortable(s_full + sl, (uint32_t)((t >> 1) & 1), abort_flag));
-      if (!ok) break;
-      tc::fence_after_sync();
-      const bool is_i8 = t < n_rest;
-      const float esc = is_i8 ? qs : p.sml;                  // > 0
-      const float4* ks4 = reinterpret_cast<const float4*>(smem + TcSmem::Ks + ks_slot * kKsBytes);
-      const float4* kb4 = ks4 + 16 + 16 * h;
-      if (is_i8 && ++ks_slot == kKsSlots) ks_slot = 0;
-      uint32_t mlo = 0u, mhi = 0u;                           // BF16 tiles: bit c set = column c (of 64) is masked
-      if (!is_i8) {
-        int lim;                                             // columns <= lim are visible
-        if (t < n_rest + n_vert) lim = min(64, nvh - (t - n_rest) * 64) - 1;
-        else lim = min(row, p.N - 1) - (wla + (t - n_rest - n_vert) * 64);
-        mlo = lim >= 31 ? 0u : lim < 0 ? 0xFFFFFFFFu : (0xFFFFFFFFu << (lim + 1));
-        mhi = lim >= 63 ? 0u : lim < 32 ? 0xFFFFFFFFu : (0xFFFFFFFFu << (lim - 31));
-      }
-      // One fused pass per tile: score -> exponent units -> 2^(y - mu) against the reference maximum as it
-      // stands -> row sum and bf16 P, two columns per instruction where the hardware has packed fp32 forms.
-      // The row maximum is not computed: a P value above 2^8 would show in the row sum of the tile, which
-      // is then > 2^8.  Only then (and for a row's first finite scores) the scores are read from tensor
-      // memory again, the maximum is taken, O is rescaled, the reference moves and the pass is repeated.
-      if constexpr (kFp8) {
-        // FP8 P V: the exact running maximum is part of the arithmetic (P~ must not pass 448), so the tile's row
-        // maximum is taken first; a row whose maximum grows goes through the out-of-line path, which rescales O.
-        uint32_t pk8[16];
-        float lsum;
-        bool grow;
-        {
-          uint32_t sr[64];
-          tc::tmem_ld32(lane_base + colS + slot * 64, *reinterpret_cast<uint32_t(*)[32]>(&sr[0]));
-          tc::tmem_ld32(lane_base + colS + slot * 64 + 32, *reinterpret_cast<uint32_t(*)[32]>(&sr[32]));
-          tc::tmem_wait_ld();
-          float* y = reinterpret_cast<float*>(sr);            // the scores in exponent units, in place
-          float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-          if (is_i8) {
-#pragma unroll
-            for (int c4 = 0; c4 < 16; ++c4) {
-              const float4 kk = ks4[c4], bb = kb4[c4];
-              const float kv[4] = {kk.x, kk.y, kk.z, kk.w}, bv[4] = {bb.x, bb.y, bb.z, bb.w};
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                y[4 * c4 + e] = fmaf(__int_as_float((int)sr[4 * c4 + e] + 0x4B400000), kv[e], bv[e]) * esc;
-                mx4[e] = fmaxf(mx4[e], y[4 * c4 + e]);
-              }
-            }
-          } else {
-#pragma unroll
-            for (int c = 0; c < 64; ++c) {
-              const uint32_t mw = c < 32 ? mlo : mhi;
-              y[c] = ((mw >> (c & 31)) & 1u) ? -INFINITY : y[c] * esc;
-              mx4[c & 3] = fmaxf(mx4[c & 3], y[c]);
-            }
-          }
-          const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-          grow = mx > m_ref;                                   // also true for a row's first finite maximum
-          const float off = kFp8Offset - (m_ref == -INFINITY ? 0.f : m_ref);
-          float rs[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-          for (int c = 0; c < 64; c += 4) {
-            const float p0 = ex2f(y[c] + off), p1 = ex2f(y[c + 1] + off), p2 = ex2f(y[c + 2] + off), p3 = ex2f(y[c + 3] + off);
-            rs[0] += p0; rs[1] += p1; rs[2] += p2; rs[3] += p3;
-            pk8[c >> 2] = tc::pack_e4m3x4(p0, p1, p2, p3);
-          }
-          lsum = (rs[0] + rs[1]) + (rs[2] + rs[3]);
-        }
-        if (__any_sync(0xffffffffu, grow)) {
-          const bool wait_pv = t > 0;
-          const TcSlowResult sr2 = tc_slow_tile<true>(lane_base + colS + slot * 64, lane_base + colO, ks4, kb4, is_i8, esc, mlo, mhi, m_ref, l,
-                                                      wait_pv ? pv_done + 2 * h + ((t - 1) & 1) : nullptr, (uint32_t)(((t - 1) >> 1) & 1),
-                                                      abort_flag);
-          ok = sr2.ok;
-          if (!ok) break;
-          m_ref = sr2.m_ref;
-          l = sr2.l;
+    if constexpr (kFp8) {
+      // The scores of a tile.  tcgen05.ld is asynchronous: the next tile's are asked for as soon as this tile's registers
+      // are free (P is packed), so that the load runs under the store of P and the hand-over.
+      uint32_t sr[64];
+      auto load_scores = [&](int t) {
+        tc::fence_after_sync();
+        tc::tmem_ld32(lane_base + colS + (t & 1) * 64, *reinterpret_cast<uint32_t(*)[32]>(&sr[0]));
+        tc::tmem_ld32(lane_base + colS + (t & 1) * 64 + 32, *reinterpret_cast<uint32_t(*)[32]>(&sr[32]));
+      };
+      auto fetch = [&](int t) {        // wait for the scores of tile t and ask for them
+        ok = __all_sync(0xffffffffu, tc::mbar_wait_abortable(s_full + 2 * h + (t & 1), (uint32_t)((t >> 1) & 1), abort_flag));
+        if (ok) load_scores(t);
+      };
+      auto tile = [&](int t, auto int8_tile) {
+        constexpr bool kI8 = decltype(int8_tile)::value;
+        const uint32_t tS = lane_base + colS + (t & 1) * 64;
+        const float esc = kI8 ? qs : p.sml;                    // > 0
+        const float4* ks4 = reinterpret_cast<const float4*>(smem + TcSmem::Ks + ks_slot * kKsBytes);
+        const float4* kb4 = ks4 + 16 + 16 * h;
+        uint32_t mlo = 0u, mhi = 0u;                           // BF16 tiles: bit c set = column c (of 64) is masked
+        if constexpr (kI8) {
+          if (++ks_slot == kKsSlots) ks_slot = 0;
         } else {
-          l += lsum;
-          // P~ as e4m3 over the first 16 columns of the S buffer just read: row r in lane r, keys 4c .. 4c+3 in column c
-          tc::tmem_st16(lane_base + colS + slot * 64, pk8);
-          tc::tmem_wait_st();
+          int lim;                                             // columns <= lim are visible
+          if (t < n_rest + n_vert) lim = min(64, nvh - (t - n_rest) * 64) - 1;
+          else lim = min(row, p.N - 1) - (wla + (t - n_rest - n_vert) * 64);
+          mlo = lim >= 31 ? 0u : lim < 0 ? 0xFFFFFFFFu : (0xFFFFFFFFu << (lim + 1));
+          mhi = lim >= 63 ? 0u : lim < 32 ? 0xFFFFFFFFu : (0xFFFFFFFFu << (lim - 31));
         }
-      } else {
+        tc::tmem_wait_ld();
+        tc::tie64(sr);
+        float* y = reinterpret_cast<float*>(sr);
+        // scores before the row's factor `esc` (INT8: s32 -> fp32 by the magic-number add, key scale and bias in one
+        // packed fma; BF16 tiles: masked columns -inf)
+        if constexpr (kI8) {
+#pragma unroll
+          for (int c4 = 0; c4 < 16; ++c4) {
+            const float4 kk = ks4[c4], bb = kb4[c4];
+            const float2 a01 = make_float2(__int_as_float((int)sr[4 * c4] + 0x4B400000), __int_as_float((int)sr[4 * c4 + 1] + 0x4B400000));
+            const float2 a23 = make_float2(__int_as_float((int)sr[4 * c4 + 2] + 0x4B400000), __int_as_float((int)sr[4 * c4 + 3] + 0x4B400000));
+            const float2 x01 = ffma2(a01, make_float2(kk.x, kk.y), make_float2(bb.x, bb.y));
+            const float2 x23 = ffma2(a23, make_float2(kk.z, kk.w), make_float2(bb.z, bb.w));
+            y[4 * c4] = x01.x; y[4 * c4 + 1] = x01.y; y[4 * c4 + 2] = x23.x; y[4 * c4 + 3] = x23.y;
+          }
+        } else if (__any_sync(0xffffffffu, mhi != 0u)) {       // mhi == 0 only if no column is masked
+#pragma unroll
+          for (int c = 0; c < 64; ++c)
+            if (((c < 32 ? mlo : mhi) >> (c & 31)) & 1u) y[c] = -INFINITY;
+        }
+        // FP8 P V: the exact running maximum is part of the arithmetic (P~ must not pass 448), so the reference moves
+        // whenever the row's maximum grows, before the tile's P~ is formed: the warp waits for P V and rescales O.  (With
+        // the pass repeated out of line for such tiles - at 16K two of five, counting all 32 rows of a warp - a
+        // call took 5.40 ms instead of 3.12.)
+        float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+        for (int c = 0; c < 64; ++c) mx4[c & 3] = fmaxf(mx4[c & 3], y[c]);
+        const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * esc;
+        const bool grow = mx > m_ref;                        // also true for a row's first finite maximum
+        if (__any_sync(0xffffffffu, grow)) {
+          const float alpha = grow ? (m_ref == -INFINITY ? 0.f : ex2f(m_ref - mx)) : 1.f;
+          ok = t == 0 || tc_rescale_o(lane_base + colO, alpha, pv_done + 2 * h + ((t - 1) & 1), (uint32_t)(((t - 1) >> 1) & 1), abort_flag);
+          if (!ok) return;
+          if (grow) { l *= alpha; m_ref = mx; }
+        }
+        const float mu = m_ref == -INFINITY ? 0.f : m_ref, off = kFp8Offset - mu;
+        const float2 esc2 = make_float2(esc, esc), off2 = make_float2(off, off);
+#pragma unroll
+        for (int c2 = 0; c2 < 32; ++c2) {
+          const float2 z = ffma2(make_float2(y[2 * c2], y[2 * c2 + 1]), esc2, off2);
+          y[2 * c2] = z.x; y[2 * c2 + 1] = z.y;
+        }
+#pragma unroll
+        for (int c = 0; c < 64; ++c) y[c] = ex2f(y[c]);
+        float2 rs4[4] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll
+        for (int c2 = 0; c2 < 32; ++c2) rs4[c2 & 3] = fadd2(rs4[c2 & 3], make_float2(y[2 * c2], y[2 * c2 + 1]));
+        const float2 rs2 = fadd2(fadd2(rs4[0], rs4[2]), fadd2(rs4[1], rs4[3]));
+        const float lsum = rs2.x + rs2.y;
+        uint32_t pk[16];
+#pragma unroll
+        for (int c = 0; c < 64; c += 4) pk[c >> 2] = tc::pack_e4m3x4(y[c], y[c + 1], y[c + 2], y[c + 3]);
+        l += lsum;
+        // sr is free: if the next scores are there already, their load runs under the hand-over of P
+        const bool early = t + 1 < n_tiles &&
+                           __all_sync(0xffffffffu, mbar_test_wait(s_full + 2 * h + ((t + 1) & 1), (uint32_t)(((t + 1) >> 1) & 1)));
+        if (early) load_scores(t + 1);
+        // P~ as e4m3 over the first 16 columns of the S buffer just read: row r in lane r, keys 4c .. 4c + 3 in column c
+        tc::tmem_st16(tS, pk);
+        tc::tmem_wait_st();
+        tc::fence_before_sync();
+        tc::mbar_arrive(p_ready + 2 * h + (t & 1));
+        if (!early && t + 1 < n_tiles) fetch(t + 1);
+      };
+      if (n_tiles > 0) fetch(0);
+      int t = 0;
+      for (; ok && t < n_rest && t < n_tiles; ++t) tile(t, TcTrue{});
+      for (; ok && t < n_tiles; ++t) tile(t, TcFalse{});
+    } else {
+      // (Asking for the next scores early, as above, was measured slower here: 9.37 against 9.25 ms at 32K.  So were two
+      // threads per row, sixteen softmax warps in all: 10.1 ms - the loop lives on shared-memory bandwidth, of which
+      // the key scales and biases of 256 rows take 1024 clocks of some 2200 per pair of tiles and the operands of
+      // the products 640, and on the issuing warps' latency, which more warps lengthen.)
+      for (int t = 0; t < n_tiles; ++t) {
+        const int slot = t & 1, sl = 2 * h + slot;
+        ok = __all_sync(0xffffffffu, tc::mbar_wait_abortable(s_full + sl, (uint32_t)((t >> 1) & 1), abort_flag));
+        if (!ok) break;
+        tc::fence_after_sync();
+        const bool is_i8 = t < n_rest;
+        const float esc = is_i8 ? qs : p.sml;                  // > 0
+        const float4* ks4 = reinterpret_cast<const float4*>(smem + TcSmem::Ks + ks_slot * kKsBytes);
+        const float4* kb4 = ks4 + 16 + 16 * h;
+        if (is_i8 && ++ks_slot == kKsSlots) ks_slot = 0;
+        uint32_t mlo = 0u, mhi = 0u;                           // BF16 tiles: bit c set = column c (of 64) is masked
+        if (!is_i8) {
+          int lim;                                             // columns <= lim are visible
+          if (t < n_rest + n_vert) lim = min(64, nvh - (t - n_rest) * 64) - 1;
+          else lim = min(row, p.N - 1) - (wla + (t - n_rest - n_vert) * 64);
+          mlo = lim >= 31 ? 0u : lim < 0 ? 0xFFFFFFFFu : (0xFFFFFFFFu << (lim + 1));
+          mhi = lim >= 63 ? 0u : lim < 32 ? 0xFFFFFFFFu : (0xFFFFFFFFu << (lim - 31));
+        }
+        // One fused pass per tile: score -> exponent units -> 2^(y - mu) against the reference maximum as it
+        // stands -> row sum and bf16 P, two columns per instruction where the hardware has packed fp32 forms.
+        // The row maximum is not computed: a P value above 2^8 would show in the row sum of the tile, which
+        // is then > 2^8.  Only then (and for a row's first finite scores) the scores are read from tensor
+        // memory again, the maximum is taken, O is rescaled, the reference moves and the pass is repeated.
         uint32_t pk[32];
         float lsum;
         {
@@ -529,7 +579,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap mQi, const __grid_constant
               pk[c2] = *reinterpret_cast<uint32_t*>(&h0);
             }
           } else {
-  #pragma unroll
+#pragma unroll
             for (int c2 = 0; c2 < 32; ++c2) {
               const uint32_t mw = c2 < 16 ? mlo : mhi;
               float2 y = ffma2(make_float2(__uint_as_float(sr[2 * c2]), __uint_as_float(sr[2 * c2 + 1])), esc2, nmu2);
@@ -547,7 +597,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap mQi, const __grid_constant
         if (__any_sync(0xffffffffu, need)) {
           // out of line: the maximum, the move of the reference and the tile's P against the new reference
           const bool wait_pv = t > 0;
-          const TcSlowResult sr2 = tc_slow_tile<false>(lane_base + colS + slot * 64, lane_base + colO, ks4, kb4, is_i8, esc, mlo, mhi, m_ref, l,
+          const TcSlowResult sr2 = tc_slow_tile(lane_base + colS + slot * 64, lane_base + colO, ks4, kb4, is_i8, esc, mlo, mhi, m_ref, l,
                                                 wait_pv ? pv_done + 2 * h + ((t - 1) & 1) : nullptr, (uint32_t)(((t - 1) >> 1) & 1),
                                                 abort_flag);
           ok = sr2.ok;
@@ -560,9 +610,9 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap mQi, const __grid_constant
           tc::tmem_st32(lane_base + colS + slot * 64, pk);
           tc::tmem_wait_st();
         }
+        tc::fence_before_sync();
+        tc::mbar_arrive(p_ready + sl);
       }
-      tc::fence_before_sync();
-      tc::mbar_arrive(p_ready + sl);
     }
     // ---- epilogue: O / l
     if (ok && n_tiles > 0)

@@ -132,6 +132,11 @@ __device__ __forceinline__ uint32_t pack_e4m3x4(float a, float b, float c, float
   return (uint32_t)lo | ((uint32_t)hi << 16);
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+// Nothing that reads r may move above this point (after a tmem_wait_ld that completes an earlier load).
+__device__ __forceinline__ void tie64(uint32_t (&r)[64]) {
+#pragma unroll
+  for (int i = 0; i < 64; ++i) asm volatile("" : "+r"(r[i]));
+}
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // One lane of a converged warp.  A warp whose 32 lanes walk a loop together and elect a lane only for the tensor

@@ -45,16 +45,19 @@ namespace hq {
 // ---- host side ---------------------------------------------------------------
 
 // Tensor map of the code planes as {unit bytes (in 8-byte elements, so that a whole unit of up to 2 KB is one row of
-// the box), units per plane, planes}, box {unit, 1, 2}, no swizzle.  The last few maps are kept (a cache's buffers change only when it grows), since encoding one costs about as much
-// host time as the launch.
+// the box), units per plane, planes}, box {unit, 1, 2}, no swizzle.  Maps are kept by what they are made of (a
+// cache's buffers change only when it grows), since encoding one costs about as much host time as the launch.
 static int kv_tensor_map(CUtensorMap* out, const void* base, int row_bytes, int64_t plane_tokens, int64_t planes, int unit_tokens) {
   struct Entry { const void* base; int row; int64_t tokens, planes; int unit; CUtensorMap map; };
-  constexpr int kKeep = 8;
+  // one place per cache of a model's layers: with eight places in turn a model of 32 layers encoded a map on every call
+  constexpr int kKeep = 128;
   static thread_local Entry kept[kKeep];
-  static thread_local int next = 0;
-  for (int i = 0; i < kKeep; ++i)
-    if (kept[i].base == base && kept[i].row == row_bytes && kept[i].tokens == plane_tokens && kept[i].planes == planes &&
-        kept[i].unit == unit_tokens) { *out = kept[i].map; return HQ_OK; }
+  const uint64_t mixed = (uint64_t)(uintptr_t)base * 0x9E3779B97F4A7C15ull;
+  Entry& e = kept[mixed >> 57];
+  if (e.base == base && e.row == row_bytes && e.tokens == plane_tokens && e.planes == planes && e.unit == unit_tokens) {
+    *out = e.map;
+    return HQ_OK;
+  }
   tc::EncodeTiledFn fn = tc::encode_fn();
   HQ_REQUIRE(fn != nullptr, HQ_ERR_CUDA, "hq_decode_splitk: cuTensorMapEncodeTiled is not available from this driver");
   const cuuint64_t unit_bytes = (cuuint64_t)row_bytes * (cuuint64_t)unit_tokens;
@@ -67,8 +70,7 @@ static int kv_tensor_map(CUtensorMap* out, const void* base, int row_bytes, int6
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   HQ_REQUIRE(r == CUDA_SUCCESS, HQ_ERR_CUDA, "hq_decode_splitk: cuTensorMapEncodeTiled failed with %d (row %d, %lld tokens, %lld planes)",
              (int)r, row_bytes, (long long)plane_tokens, (long long)planes);
-  kept[next] = Entry{base, row_bytes, plane_tokens, planes, unit_tokens, *out};
-  next = (next + 1) % kKeep;
+  e = Entry{base, row_bytes, plane_tokens, planes, unit_tokens, *out};
   return HQ_OK;
 }
 

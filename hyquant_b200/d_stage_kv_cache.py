@@ -288,6 +288,47 @@ class DStageLayerCache:
         p.args.lengths = None if self._lengths is None else self._lengths.data_ptr()
         return p
 
+    def _plain_launch(self, query_states: torch.Tensor, kv_repeat: int, out: Optional[torch.Tensor],
+                      key_states: Optional[torch.Tensor] = None, value_states: Optional[torch.Tensor] = None):
+        """The launch of the everyday call - a plan that has been launched before, bf16 rows that lie one behind the other
+        - without the views and checks of the general route (which cost more host time than the launch itself).
+        Returns the output, or None if the call is not of that kind; nothing has happened then."""
+        p = self._plan
+        bf16 = torch.bfloat16
+        if (p is None or self._plan_fresh or p.kv_repeat != kv_repeat or query_states.dtype != bf16
+                or query_states.shape != (self._B, self._H_KV * kv_repeat, 1, 128) or not query_states.is_contiguous()):
+            return None
+        q_ptr = query_states.data_ptr()
+        if q_ptr & 7 or query_states.device != p.device:
+            return None
+        if out is not None and (out.dtype != bf16 or out.shape != query_states.shape or not out.is_contiguous()):
+            return None
+        a = p.args
+        if key_states is not None:
+            kv_shape = (self._B, self._H_KV, 1, 128)
+            if (key_states.dtype != bf16 or value_states.dtype != bf16 or key_states.shape != kv_shape
+                    or value_states.shape != kv_shape or not key_states.is_contiguous() or not value_states.is_contiguous()):
+                return None
+            k_ptr, v_ptr = key_states.data_ptr(), value_states.data_ptr()
+            if (k_ptr | v_ptr) & 15 or not key_states.is_cuda or not value_states.is_cuda:
+                return None
+        if out is None:
+            out = torch.empty_like(query_states, memory_format=torch.contiguous_format)
+        stream = _lib.stream_ptr(p.device)
+        if key_states is not None:
+            a.k_new, a.v_new, a.kn_stride, a.vn_stride = k_ptr, v_ptr, 128, 128
+        a.n_quant, a.n_staging = self._n_quant, self._staging_ptr
+        a.lengths = None if self._lengths is None else self._lengths.data_ptr()
+        a.q, a.q_stride, a.out, a.out_stride, a.out_dtype = q_ptr, 128, out.data_ptr(), 128, _lib.HQ_BF16
+        a.peer_world = 0
+        a.partial_m = a.partial_l = a.partial_acc = None
+        rc = p._fn(p._args_ref, stream)
+        if key_states is not None:
+            a.k_new = a.v_new = None
+        if rc != 0:
+            _lib.check(rc, "hq_decode_splitk")
+        return out
+
     def decode_attention(self, query_states: torch.Tensor, kv_repeat: int, *, partial=None,
                          out: Optional[torch.Tensor] = None, peer=None) -> torch.Tensor:
         """Attention of one new token over the four segments (reference :219-303).
@@ -296,6 +337,10 @@ class DStageLayerCache:
         ``partial=(m, l, acc)`` requests the un-normalised softmax state instead
         (sequence-sharded decode).  ``out`` (not in the reference): a [B, H_Q, 1, D] tensor with
         contiguous rows to write into instead of a new one."""
+        if partial is None and peer is None:
+            res = self._plain_launch(query_states, kv_repeat, out)
+            if res is not None:
+                return res
         B_, H_Q_, _, D_ = query_states.shape
         q2d = query_states.reshape(B_ * H_Q_, D_)
         plan = self._decode_plan(q2d, kv_repeat)
@@ -322,6 +367,12 @@ class DStageLayerCache:
         ``rope=(cos, sin)`` (not in the reference, whose patched forwards rotate q and k with separate eager kernels before
         the cache, src/patch/patch_llama.py:58-65): bf16 ``[B, D]`` or ``[B, 1, D]`` rotary factors of this step's position;
         ``query_states`` and ``key_states`` are then given UNROTATED and the kernel rotates them itself."""
+        if rope is None and partial is None and peer is None and self._staging_ptr < GROUP_SIZE - 1:
+            res = self._plain_launch(query_states, kv_repeat, out, key_states, value_states)
+            if res is not None:
+                self._staging_ptr += 1
+                self._seq_len += 1
+                return res
         B, H_KV, S, D = key_states.shape
         cos = sin = None
         if rope is not None:

@@ -225,6 +225,7 @@ class DecodePlan:
         self.ws = decode_workspace(q.device, self.BH_KV, kv_repeat)
         a.workspace, a.workspace_bytes = self.ws.data_ptr(), self.ws.numel()
         self.args = a
+        self._args_ref = C.byref(a)
         self._keep = keep
         self._fn = _lib.lib().hq_decode_splitk
 

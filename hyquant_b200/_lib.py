@@ -15,6 +15,7 @@ LIB_PATH = os.path.join(PKG, "libhyquant_b200.so")
 
 HQ_BF16, HQ_F16, HQ_F32 = 0, 1, 2
 HQ_DECODE_OVERLAP_PREVIOUS = 1
+HQ_DECODE_SHARED_CHIP = 2
 HQ_OK = 0
 ERR_NAMES = {-1: "HQ_ERR_INVALID", -2: "HQ_ERR_UNSUPPORTED", -3: "HQ_ERR_ALIGNMENT",
              -4: "HQ_ERR_WORKSPACE", -5: "HQ_ERR_CUDA", -6: "HQ_ERR_TIMEOUT"}

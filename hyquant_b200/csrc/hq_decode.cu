@@ -152,8 +152,10 @@ extern "C" int hq_decode_splitk(const hq_decode_args* a, void* stream) {
                  "hq_decode_splitk: BF16 segment %d must be 16-byte aligned with head strides multiple of 8", s);
     }
   }
-  HQ_REQUIRE((a->flags & ~HQ_DECODE_OVERLAP_PREVIOUS) == 0, HQ_ERR_INVALID, "hq_decode_splitk: unknown flags 0x%x", a->flags);
+  HQ_REQUIRE((a->flags & ~(HQ_DECODE_OVERLAP_PREVIOUS | HQ_DECODE_SHARED_CHIP)) == 0, HQ_ERR_INVALID, "hq_decode_splitk: unknown flags 0x%x",
+             a->flags);
   p.overlap = (a->flags & HQ_DECODE_OVERLAP_PREVIOUS) ? 1 : 0;
+  p.shared = (a->flags & HQ_DECODE_SHARED_CHIP) ? 1 : 0;
   p.R = a->kv_repeat;
   p.out_dtype = a->out_dtype;
   p.sml = a->sm_scale * 1.44269504f;

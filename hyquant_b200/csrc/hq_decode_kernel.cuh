@@ -20,7 +20,9 @@ namespace hq {
 #ifndef HQ_DEC_WARPS2
 #define HQ_DEC_WARPS2 12
 #endif
-__host__ __device__ constexpr int warps_of(int NT) { return NT == 2 ? HQ_DEC_WARPS2 : HQ_DEC_WARPS1; }
+// A launch that shares the chip with others (kMode 3, other branches of a graph) takes half as many warps a CTA and two
+// CTAs an SM: one CTA's prologue and merge then run under the other's main loop.
+__host__ __device__ constexpr int warps_of(int NT, int mode = 0) { return (NT == 2 ? HQ_DEC_WARPS2 : HQ_DEC_WARPS1) / (mode == 3 ? 2 : 1); }
 constexpr int kSlots = 3;
 constexpr int kScaleLanes = 8;            // lanes of a warp that fetch a unit's scales (16 bytes each)
 // quantised tokens per unit: 32, or 16 when 32 rows of K and V codes would not fit the 4 KB of a BF16 unit (every pair
@@ -59,6 +61,7 @@ struct DecodeParams {
   __nv_bfloat16* stage_k; __nv_bfloat16* stage_v;   // staging buffers, written only when the call carries a new token
   int scale_tma;                          // scales ride in the bulk copies (aligned rows) or are loaded directly
   int kv_fused;                           // K and V codes of a head are two planes of one tensor: one request per unit
+  int shared;                             // other launches run beside this one: half-size CTAs (kMode 3)
   int overlap;                            // launched with programmatic stream serialisation
   const int* lengths;                     // device {n_quant, n_staging} overriding the values above (or null)
   const __nv_bfloat16* rope_cos; const __nv_bfloat16* rope_sin;   // [batch, 128] rotary factors of the step (or null)
@@ -411,14 +414,15 @@ __device__ __forceinline__ float ld_cluster_f32(uint32_t addr, int rank) {
 
 // kMode: 0 = the splits of a head merge through the workspace; 1 = the same, followed by the exchange with the other
 // sequence shards over peer memory; 2 = the splits of a head are one thread-block cluster and merge through
-// distributed shared memory.  Instantiated apart, so that each form costs the others no registers.
+// distributed shared memory; 3 = as 0 with half the warps, two CTAs an SM.  Instantiated apart, so that each form costs
+// the others no registers.
 template <int NT, bool kScaleTma, int KB, int VB, int kMode>
-__global__ void __launch_bounds__(warps_of(NT) * 32, 1)
+__global__ void __launch_bounds__(warps_of(NT, kMode) * 32, kMode == 3 ? 2 : 1)
 decode_splitk_kernel(const __grid_constant__ CUtensorMap kv_map, const DecodeParams p) {
   constexpr bool kPeer = kMode == 1, kCluster = kMode == 2;
   using F = Fmt<KB, VB>;
   using VF = VFmt<VB>;
-  constexpr int kWarps = warps_of(NT), kThreads = kWarps * 32;
+  constexpr int kWarps = warps_of(NT, kMode), kThreads = kWarps * 32;
   constexpr int kSlotBytes = F::kSlot, kUnitQ = F::kUnitQ, kChunks = F::kChunks;
   constexpr int kQItems = NT * 8;                                   // (tile, head) pairs whose query row is loaded
   constexpr int kQIter = (kQItems + kWarps - 1) / kWarps;           // per warp: items warp, warp + kWarps, ...
@@ -1245,14 +1249,14 @@ decode_splitk_kernel(const __grid_constant__ CUtensorMap kv_map, const DecodePar
 
 // ---- launch ------------------------------------------------------------------
 
-static size_t decode_smem_bytes(int NT, int slot_bytes) {
-  const int w = warps_of(NT);
+static size_t decode_smem_bytes(int NT, int slot_bytes, int mode) {
+  const int w = warps_of(NT, mode);
   return (size_t)w * kSlots * slot_bytes + (size_t)NT * 512 * 4 * 2 + (size_t)NT * 8 * 4 + (size_t)w * kSlots * 8;
 }
 
 template <int NT, bool kScaleTma, int KB, int VB, int kMode>
 static int launch_decode(const DecodeParams& p, const CUtensorMap& kv_map, dim3 grid, cudaStream_t st, int* clusters_out) {
-  const size_t smem = decode_smem_bytes(NT, Fmt<KB, VB>::kSlot);
+  const size_t smem = decode_smem_bytes(NT, Fmt<KB, VB>::kSlot, kMode);
   static thread_local int attr_dev = -1;
   int dev = 0;
   HQ_CUDA(cudaGetDevice(&dev));
@@ -1263,7 +1267,7 @@ static int launch_decode(const DecodeParams& p, const CUtensorMap& kv_map, dim3 
   }
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
-  cfg.blockDim = dim3(warps_of(NT) * 32);
+  cfg.blockDim = dim3(warps_of(NT, kMode) * 32);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute attr[2];
@@ -1316,6 +1320,8 @@ static int launch_decode_bits(const DecodeParams& p, const CUtensorMap& kv_map, 
     if (!p.scale_tma) { if (clusters_out) *clusters_out = 0; return clusters_out ? HQ_OK : HQ_ERR_INVALID; }
     return NT == 1 ? launch_decode<1, true, KB, VB, 2>(p, kv_map, grid, st, clusters_out) : launch_decode<2, true, KB, VB, 2>(p, kv_map, grid, st, clusters_out);
   }
+  if (p.shared && p.scale_tma)
+    return NT == 1 ? launch_decode<1, true, KB, VB, 3>(p, kv_map, grid, st, clusters_out) : launch_decode<2, true, KB, VB, 3>(p, kv_map, grid, st, clusters_out);
   if (NT == 1) return p.scale_tma ? launch_decode<1, true, KB, VB, 0>(p, kv_map, grid, st, clusters_out) : launch_decode<1, false, KB, VB, 0>(p, kv_map, grid, st, clusters_out);
   return p.scale_tma ? launch_decode<2, true, KB, VB, 0>(p, kv_map, grid, st, clusters_out) : launch_decode<2, false, KB, VB, 0>(p, kv_map, grid, st, clusters_out);
 }

@@ -432,9 +432,10 @@ class DStageLayerCache:
                             overlap: bool = True, num_splits: int = 0, workspace: Optional[torch.Tensor] = None):
         """Issue the fused ``decode_step`` launch WITHOUT counting the token: for use inside a CUDA-graph capture
         (lengths bound with :meth:`bind_lengths`; every tensor argument must keep its address across replays).
-        After each replay call :meth:`count_replayed_step`.  ``num_splits`` (0 = chosen for this launch alone) and
-        ``workspace`` (split-K scratch, ``hq_decode_workspace_bytes``, zero-filled; kept by the caller): for launches
-        that share the chip with others on other branches of the graph."""
+        After each replay call :meth:`count_replayed_step`.  ``num_splits`` (0 = chosen for this launch alone; else the
+        launch takes half-size blocks, ``HQ_DECODE_SHARED_CHIP``) and ``workspace`` (split-K scratch,
+        ``hq_decode_workspace_bytes``, zero-filled; kept by the caller): for launches that share the chip with others on
+        other branches of the graph."""
         if self._lengths is None:
             raise HyQuantError("bind_lengths first: a captured launch must not carry the lengths in its arguments")
         B, H_KV, S, D = key_states.shape
@@ -447,6 +448,8 @@ class DStageLayerCache:
         a.flags = _lib.HQ_DECODE_OVERLAP_PREVIOUS if (overlap and self.k_bits == 4 and self.v_bits == 4) else 0
         a.k_new, a.v_new, a.kn_stride, a.vn_stride = k2.data_ptr(), v2.data_ptr(), k2.stride(0), v2.stride(0)
         a.num_splits = num_splits
+        if num_splits > 0:
+            a.flags |= _lib.HQ_DECODE_SHARED_CHIP
         if workspace is not None:
             a.workspace, a.workspace_bytes = workspace.data_ptr(), workspace.numel()
         try:

@@ -51,22 +51,25 @@ class DecodeStepGraph:
         self._ws, self._streams = [], []         # one split-K workspace per branch of the graph, and the branches' streams
         self._warm = False
 
-    BRANCHES = 8
+    BRANCHES = 16
 
     def _plan_launches(self):
         """(splits of a head, branches of the graph; 0 splits = as a launch that has the chip for itself).
 
-        Eight branches: a finished launch's place is taken at once by another branch's blocks, while sixteen or thirty-two
-        measured within 5 % of eight.  Splits: as many as give the launches in flight about 1.75 blocks per SM (a block
-        fills an SM's shared memory, so a part of them waits and takes over where others end).  Measured on 8 kv-heads,
-        with 1 / 2 / 4 / 18 splits: 32 layers of an 8K prefix 204 / 154 / 144 / 266 us, 16 layers of 16K 174 / 119 /
-        122 / 182, 32 layers of 1K 90 / 126 / 90 / 210, 8 layers of 2K 63 / 47 / 48 / 76; one launch after the other with
-        18 splits each: 345 us for 32 layers of 8K."""
+        The launches share the chip, so they run as half-size blocks, two to an SM (HQ_DECODE_SHARED_CHIP).  Splits: as many
+        as give sixteen launches in flight about 1.75 blocks per place (some wait and take over where others end), or, with
+        few layers, one block per place; and no more than leave a warp four units (32 quantised or 8 BF16 tokens) to
+        work on.  Measured on 8 kv-heads: 32 layers of an 8K prefix 126 us with 4 splits (16 branches of full-size
+        blocks 143 to 165, one launch after the other 345), 16 layers of 16K 111 with 4 (115), 32 layers of 1K 75 with 2 to 4
+        (82), 8 layers of 2K 43 with 2 to 4 (48)."""
         branches = min(self.BRANCHES, len(self.layers))
         if branches == 1:
             return 0, 1
         sms = torch.cuda.get_device_properties(self.dev_in.device).multi_processor_count
-        return max(1, min(18, round(1.75 * sms / (branches * self.B * self.H_KV)))), branches
+        heads, layer = self.B * self.H_KV, self.layers[0]
+        units = layer._n_quant // 32 + (layer.k_topk.shape[1] + layer.k_window.shape[1] + layer._staging_ptr) // 8
+        wanted = max(round(3.5 * sms / (self.BRANCHES * heads)), 2 * sms // (len(self.layers) * heads))
+        return max(1, min(18, wanted, units // 32)), branches
 
     def _eager(self):
         self.dev_in.copy_(self.host_in, non_blocking=True)
@@ -76,7 +79,7 @@ class DecodeStepGraph:
 
     def _capture(self):
         # Every layer's rows are in the message, so the layers do not wait for one another: their launches are captured on
-        # several branches that fork behind the input copy and join before the output copy, each branch with a split-K
+        # sixteen branches that fork behind the input copy and join before the output copy, each branch with a split-K
         # workspace of its own (a branch's launches follow one another).  A layer is then cut into fewer, longer
         # blocks, because the other layers fill the chip.
         splits, branches = self._plan_launches()

@@ -105,6 +105,9 @@ int hq_staging_append(const void* k_new, const void* v_new, int64_t k_stride, in
  * of q, the previous decode call).  The caller promises that it writes nothing else of this
  * call's cache: not the older prefix, nor the vertical-line and window segments. */
 #define HQ_DECODE_OVERLAP_PREVIOUS 1
+/* Other launches run beside this one (branches of a graph, other streams): the kernel takes CTAs of half the size, two to
+ * an SM, where it has that form (16-byte aligned scale rows, no peers).  Give num_splits with it. */
+#define HQ_DECODE_SHARED_CHIP 2
 
 typedef struct hq_decode_args {
   int32_t struct_bytes;        /* sizeof(hq_decode_args), checked */
@@ -118,7 +121,7 @@ typedef struct hq_decode_args {
   int32_t out_dtype;           /* HQ_BF16 / HQ_F16 / HQ_F32 */
   int32_t num_splits;          /* 0 = choose automatically */
   float   sm_scale;            /* softmax scale, e.g. head_dim^-0.5 */
-  int32_t flags;               /* 0, or HQ_DECODE_OVERLAP_PREVIOUS */
+  int32_t flags;               /* 0, or HQ_DECODE_* bits */
   int32_t k_bits;              /* bit width of the quantised K prefix: 8, 4 or 2 (0 = 4) */
   int32_t v_bits;              /* the same for V; every pair is one instantiation of the same kernel */
   const void* q;               /* bf16 [BH_KV*kv_repeat, 128] */

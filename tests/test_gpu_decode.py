@@ -217,6 +217,28 @@ def test_decode_cluster_merge_against_workspace_merge(R, heads, nq):
         assert np.all(np.abs(out - plain) <= 2e-3 + 2.0 ** -7 * np.abs(plain))
 
 
+@pytest.mark.parametrize("bits", [(kb, vb) for kb in (8, 4, 2) for vb in (8, 4, 2)])
+@pytest.mark.parametrize("R,lens", [(4, (1300, 40, 17, 128)), (16, (1300, 40, 17, 128)), (7, (33, 0, 1, 0)), (1, (0, 9, 0, 64)), (9, (4113, 206, 127, 256))])
+def test_half_size_blocks_against_full_size_blocks(bits, R, lens, monkeypatch):
+    """HQ_DECODE_SHARED_CHIP: blocks of half the warps, two to an SM.  The same units over fewer warps - only the order of
+    the fp32 sums differs - for every pair of bit widths, one and two tiles of query heads, one and more splits; rows
+    of scales that are not 16-byte aligned fall back to the full-size form."""
+    c, q = build_case(3, R, *lens, seed=R * 100 + lens[0], k_bits=bits[0], v_bits=bits[1])
+    ref = orc.decode_attention_exact(q, c, R).reshape(-1, 128)
+    plain = {s: run_gpu(c, q, R, num_splits=s) for s in (1, 3, 7)}
+    run = dd.DecodePlan.run
+
+    def shared(self, *a, **kw):
+        self.args.flags |= hq._lib.HQ_DECODE_SHARED_CHIP
+        return run(self, *a, **kw)
+
+    monkeypatch.setattr(dd.DecodePlan, "run", shared)
+    for s, want in plain.items():
+        out = run_gpu(c, q, R, num_splits=s)
+        check_close(out, ref)
+        assert np.all(np.abs(out - want) <= 2e-3 + 2.0 ** -7 * np.abs(want))
+
+
 def test_decode_split_invariance_and_partials():
     c, q = build_case(4, 4, 5000, 250, 77, 128, seed=9)
     ref = orc.decode_attention_exact(q, c, 4).reshape(-1, 128)

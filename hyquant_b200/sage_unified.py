@@ -145,7 +145,7 @@ class PrefillPlan:
         nqb, nkb = (N + 127) // 128, (N + 63) // 64
         # A window that covers the prompt leaves no INT8 tile and no vertical line (16-bit causal attention): without K
         # smoothing the BF16 operands are then q and k as they are, and nothing reads codes, scales or biases
-        # (2 x 32 heads x 1973 tokens: 54 of 189 us were spent on them).
+        # (2 x 32 heads x 1973 tokens: 58 of 189 us were spent on them).
         bf16_only = alias_inputs and window_size >= N and not smooth_k and N > 0
         if bf16_only:
             q_bf, k_bf = qb.contiguous(), kb.contiguous()

@@ -45,6 +45,7 @@ constexpr uint32_t kColS = 0, kColO = 256; // S buffer of head h, parity s: kCol
 
 constexpr int kKStages = 3;    // depth of the K ring: Q K^T runs two tiles ahead of P V and frees its slot at once
 constexpr int kVStages = 4;    // depth of the V ring
+constexpr int kNearRun = 2;    // a head waits for a K item before a due P V across at most this many items of the other head
 constexpr int kKsSlots = 6;    // ring of key-scale rows: a row is dead once P V of its item + 2 has been issued
 constexpr int kKsBytes = 768;  // 64 key scales | 64 bias terms of head A | 64 bias terms of head B
 struct TcSmem {              // offsets from a 1024-aligned base
@@ -317,11 +318,14 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap mQi, const __grid_constant
     // addresses then stay in uniform registers (the issuing loop was as long as the softmax loop when one diverged
     // lane ran it: 32K hybrid 9.98 -> 9.69 ms, FP8 16K 5.91 -> 5.38 ms, 16-bit 2 x 1973 207 -> 189 us per call).
     // In the head's own order: Q K^T of tiles 0 and 1, then for every tile t:
-    // P V of t, Q K^T of t + 2.  The S buffer that Q K^T of t + 2 overwrites held P of tile t, and the tensor
+    // P V of t, Q K^T of t + 2 (across a long run of the other head's tiles: P V of all tiles before it, then Q K^T of
+    // the next two).  The S buffer that Q K^T of t + 2 overwrites held P of tile t, and the tensor
     // core runs one thread's operations in issue order, so the scores of the next tile are ready while the
     // head's softmax threads are still on the current one.  Ring slots come back when both heads are done
     // with them: a head arrives by tcgen05.commit for an item it used and by a plain arrive for a
-    // vertical-line item of the other head, in ring order either way.
+    // vertical-line item of the other head, in ring order either way.  No wait may need something of a LATER item than
+    // the one it is for, except K of the next few: every pair of tile counts then passes (walked on the CPU with these
+    // depths by the tests).
     const int h = warp - 9;
     if (h < plan.nheads) {
       constexpr uint32_t idesc_i8 = tc::make_idesc(2, tc::kFmtS8, tc::kFmtS8, 128, 64);
@@ -371,42 +375,63 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap mQi, const __grid_constant
         tc::mma_commit(s_full + 2 * h + (tq & 1));
         tc::mma_commit(k_empty + cq.stage);
       };
-      for (int i = 0; i < 2 && i < n_t; ++i) {
-        if (ok) k_ready();
-        if (!ok) break;
-        tc::fence_after_sync();
-        if (tc::elect_one()) qk_issue();
-        ++tq;
-        cq.next(plan);
-      }
-      for (int t = 0; ok && t < n_t; ++t) {
-        // the operands first, P last: from the moment P is there nothing is waited for, and P V of t and Q K^T of t + 2
-        // are issued together (a wait costs the warp some 400 clocks even if what it waits for is there: 32K hybrid
-        // 9.27 -> 9.05 ms, 8K 867 -> 844 us)
-        const bool more = t + 2 < n_t;
-        v_ready();
-        if (ok && more) k_ready();
-        if (!ok) break;
-        const int sl = 2 * h + (t & 1);
-        ok = wait(p_ready + sl, (uint32_t)((t >> 1) & 1));
-        if (!ok) break;
-        tc::fence_after_sync();
-        const uint32_t aP = tS + 64u * (t & 1);
-        const uint64_t bV = dV + (uint64_t)(cp.stage * 1024);
-        if (tc::elect_one()) {
-          if constexpr (kFp8) {     // 64 keys = two K steps of 32 e4m3: 8 columns of P, 32 bytes of a V^T row each
-#pragma unroll
-            for (int k = 0; k < 2; ++k) tc::mma_f8_ts(tO, aP + 8 * k, bV + 2 * k, idesc_pv8, (t > 0 || k > 0) ? 1u : 0u);
-          } else {
-#pragma unroll
-            for (int k = 0; k < 4; ++k) tc::mma_bf16_ts(tO, aP + 8 * k, bV + 2 * k, idesc_pv, (t > 0 || k > 0) ? 1u : 0u);
-          }
-          tc::mma_commit(pv_done + sl);
-          tc::mma_commit(v_empty + cp.stage);
-          if (more) qk_issue();
+      // The other head's vertical-line items that K's walk still has to hand back before this head's next item, if they are
+      // more than kNearRun (where this head's list is the shorter one; in the interleaved part it is one item).
+      auto run_ahead = [&]() {
+        return cq.kind == 1 && cq.hh != h && cq.j + (h == 0 ? 1 : 0) >= plan.nvert(h) && plan.nvert(1 - h) - cq.j > kNearRun;
+      };
+      int t = 0;
+      while (ok && t < n_t) {
+        // the start, or nothing issued ahead across a run of the other head's items: both walks stand here, the run goes
+        // back K and V item by item
+        while (ok && !cq.feeds(h)) {
+          ok = wait(k_full + cq.stage, cq.par);
+          if (ok && tc::elect_one()) tc::mbar_arrive(k_empty + cq.stage);
+          ok = ok && wait(v_full + cp.stage, cp.par);
+          if (ok && tc::elect_one()) tc::mbar_arrive(v_empty + cp.stage);
+          cq.next(plan);
+          cp.next(plan);
         }
-        cp.next(plan);
-        if (more) { ++tq; cq.next(plan); }
+        for (int i = 0; ok && i < 2 && tq < n_t && (i == 0 || !run_ahead()); ++i) {
+          k_ready();
+          if (!ok) break;
+          tc::fence_after_sync();
+          if (tc::elect_one()) qk_issue();
+          ++tq;
+          cq.next(plan);
+        }
+        if (!ok) break;
+        for (; t < tq; ++t) {
+          // the operands first, P last: from the moment P is there nothing is waited for, and P V of t and Q K^T of t + 2
+          // are issued together (a wait costs the warp some 400 clocks even if what it waits for is there: 32K hybrid
+          // 9.27 -> 9.05 ms, 8K 867 -> 844 us).  Not across a run of the other head's items: that head needs the V slots
+          // which P V of t and t + 1 give back to come to the end of its run, and K of t + 2 lies behind it - the two heads
+          // would wait for one another (with rings of three and four slots: runs of five items and more).
+          const bool more = tq == t + 2 && tq < n_t && !run_ahead();
+          v_ready();
+          if (ok && more) k_ready();
+          if (!ok) break;
+          const int sl = 2 * h + (t & 1);
+          ok = wait(p_ready + sl, (uint32_t)((t >> 1) & 1));
+          if (!ok) break;
+          tc::fence_after_sync();
+          const uint32_t aP = tS + 64u * (t & 1);
+          const uint64_t bV = dV + (uint64_t)(cp.stage * 1024);
+          if (tc::elect_one()) {
+            if constexpr (kFp8) {     // 64 keys = two K steps of 32 e4m3: 8 columns of P, 32 bytes of a V^T row each
+#pragma unroll
+              for (int k = 0; k < 2; ++k) tc::mma_f8_ts(tO, aP + 8 * k, bV + 2 * k, idesc_pv8, (t > 0 || k > 0) ? 1u : 0u);
+            } else {
+#pragma unroll
+              for (int k = 0; k < 4; ++k) tc::mma_bf16_ts(tO, aP + 8 * k, bV + 2 * k, idesc_pv, (t > 0 || k > 0) ? 1u : 0u);
+            }
+            tc::mma_commit(pv_done + sl);
+            tc::mma_commit(v_empty + cp.stage);
+            if (more) qk_issue();
+          }
+          cp.next(plan);
+          if (more) { ++tq; cq.next(plan); }
+        }
       }
     }
   } else {

@@ -124,6 +124,47 @@ def test_vertical_attention_vs_dense(B, H_Q, H_KV, N, W):
         assert max_abs(to_np(out), rr) <= MAX_ABS
 
 
+def uneven_lists(B, H_Q, N, W, T):
+    """[B, H_Q, T] positions: heads in turn with all lines early, all late, spread, in the middle - every block then serves
+    two heads with up to T / 64 tiles more for the one than for the other."""
+    prefix = N - W
+    forms = [np.arange(T), prefix - T + np.arange(T), np.arange(T) * prefix // T, (prefix - T) // 2 + np.arange(T)]
+    return torch.from_numpy(np.stack([np.stack([forms[(h + b) % 4][::-1] for h in range(H_Q)]) for b in range(B)]).copy()).to(DEV)
+
+
+@pytest.mark.parametrize("H_Q,H_KV,N,W,T", [(4, 1, 2600, 128, 700), (3, 1, 1500, 64, 640), (4, 2, 2300, 0, 330), (2, 1, 3000, 256, 1900)])
+@pytest.mark.parametrize("pv_fp8", [False, True])
+def test_heads_with_unequal_numbers_of_vertical_tiles(H_Q, H_KV, N, W, T, pv_fp8):
+    q, k, v = make(1, H_Q, H_KV, N, W, N + T)
+    plan = su.PrefillPlan(t_bf16(q), t_bf16(k), t_bf16(v), uneven_lists(1, H_Q, N, W, T), W, None, True, pv_fp8=pv_fp8)
+    out = to_np(plan.run())
+    plan.check_status()
+    ref = orc.dense_causal_attention(q, k, v)
+    if pv_fp8:                                # the price of the format, as in test_gpu_fp8_pv.py
+        assert np.isfinite(out).all() and orc.rel_mse(out, ref) <= 5e-3
+    else:
+        check(out, ref)
+    # the other order of each pair of heads (a warp's rows past N are the next head's and may make it move its
+    # references earlier: whole warps of the head's own rows are compared)
+    flip = torch.arange(H_Q - 1, -1, -1, device=DEV)
+    if H_KV == 1 and H_Q % 2 == 0:
+        other = su.hybrid_prefill(t_bf16(q)[:, flip], t_bf16(k), t_bf16(v), uneven_lists(1, H_Q, N, W, T)[:, flip], W, None, True, pv_fp8=pv_fp8)
+        assert max_abs(to_np(other[:, flip])[:, :, :N // 32 * 32], out[:, :, :N // 32 * 32]) == 0
+
+
+def test_one_position_given_many_times():
+    """A list that repeats one position (as the clamp of positions past the prefix makes it) is longer than the prefix it
+    stands in: eleven tiles of one head in front of the first window tile, after one INT8 tile."""
+    q, k, v = make(1, 2, 1, 900, 64, 8)
+    idx = torch.zeros(1, 2, 700, dtype=torch.int64, device=DEV)
+    idx[0, 1] = 10 ** 6
+    plan = su.PrefillPlan(t_bf16(q), t_bf16(k), t_bf16(v), idx, 64, None, True)
+    out = to_np(plan.run())
+    plan.check_status()
+    rr = orc.hybrid_prefill_reference(q, k, v, idx.clamp(0, 900 - 64 - 1).cpu().numpy(), window_size=64, round_fn=orc.bf16_round)
+    assert np.isfinite(out).all() and max_abs(out, rr) <= MAX_ABS
+
+
 def test_plan_reuse_and_status_word():
     q, k, v = make(1, 8, 2, 900, 128, 17)
     vidx = hq.compute_vertical_indices(t_bf16(q), t_bf16(k), 128, 0.05, kv_repeat=4)

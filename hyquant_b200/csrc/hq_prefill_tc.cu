@@ -23,7 +23,8 @@
 //                      final O / l from tensor memory.
 // Tensor memory (512 columns): S_A0 | S_A1 | S_B0 | S_B1 (64 each) | O_A | O_B (128 each).
 // All shared-memory operands are K-major: V is transposed once per call by the preparation pass.
-// Every wait is bounded and abortable; a failed wait raises bit 1 of the status word.
+// Every wait is bounded and abortable; a failed wait raises bit 1 of the status word, and the rows of the block and of
+// those after it are NaN.
 #include "hq_tc05.cuh"
 
 namespace hq {
@@ -46,6 +47,7 @@ constexpr uint32_t kColS = 0, kColO = 256; // S buffer of head h, parity s: kCol
 constexpr int kKStages = 3;    // depth of the K ring: Q K^T runs two tiles ahead of P V and frees its slot at once
 constexpr int kVStages = 4;    // depth of the V ring
 constexpr int kNearRun = 2;    // a head waits for a K item before a due P V across at most this many items of the other head
+constexpr uint32_t kDrainPolls = 400000;   // limit of the waits at the end of a block
 constexpr int kKsSlots = 6;    // ring of key-scale rows: a row is dead once P V of its item + 2 has been issued
 constexpr int kKsBytes = 768;  // 64 key scales | 64 bias terms of head A | 64 bias terms of head B
 struct TcSmem {              // offsets from a 1024-aligned base
@@ -189,13 +191,23 @@ __device__ __noinline__ TcSlowResult tc_slow_tile(uint32_t tS, uint32_t tO, cons
   return res;
 }
 
+// The output rows of a block that gave up, or that was skipped after one that did: NaN, so that a caller who does not
+// read the status word (which takes a synchronisation) never takes memory nobody wrote for a result.  All threads.
+__device__ __noinline__ void tc_fill_nan(const PrefillTcParams& p, int b, int hq0, int nheads, int s0) {
+  const float nan = __int_as_float(0x7FFFFFFF);
+  for (int x = threadIdx.x; x < nheads * 128 * 128; x += kTcThreads) {
+    const int h = x >> 14, row = s0 + ((x >> 7) & 127);
+    if (row < p.N) store_out(p.out, b * p.o_sb + (hq0 + h) * p.o_sh + (int64_t)row * p.o_sn + (x & 127), nan, p.out_dtype);
+  }
+}
+
 template <bool kFp8>
 __global__ void __launch_bounds__(kTcThreads, 1)
 prefill_tc_kernel(const __grid_constant__ CUtensorMap mQi, const __grid_constant__ CUtensorMap mQb,
                   const __grid_constant__ CUtensorMap mKi, const __grid_constant__ CUtensorMap mKb,
                   const __grid_constant__ CUtensorMap mVt, const __grid_constant__ CUtensorMap mXk,
                   const __grid_constant__ CUtensorMap mXv, const __grid_constant__ CUtensorMap mKs,
-                  const __grid_constant__ CUtensorMap mKbs, const PrefillTcParams p) {
+                  const __grid_constant__ CUtensorMap mKbs, const __grid_constant__ PrefillTcParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + TcSmem::Bar);
@@ -207,14 +219,14 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap mQi, const __grid_constant
   uint64_t* s_full = v_empty + kVStages;         // [head][2]
   uint64_t* p_ready = s_full + 4;                // [head][2]
   uint64_t* pv_done = p_ready + 4;               // [head][2]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_done + 4);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(pv_done + 5);
+  uint64_t* drained = pv_done + 4;               // [head]: the head's last product is done
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drained + 2);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(drained + 3);
 
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   __shared__ int s_skip;
   if (tid == 0) s_skip = *reinterpret_cast<volatile int*>(p.status) & 2;
   __syncthreads();
-  if (s_skip) return;                         // an earlier CTA gave up: drain the grid quickly
   const int R = p.H_Q / p.H_KV, pairs = (R + 1) / 2;
   // Blocks in the order of their length, longest first, over a group of head pairs whose K and V stay in L2 together (the
   // host sizes the groups): head by head, each from its longest block to its shortest, left the SMs that took the last
@@ -229,6 +241,10 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap mQi, const __grid_constant
   const int s0 = qb * 128;
   TcPlan plan;
   plan.nheads = (2 * pr + 1 < R) ? 2 : 1;
+  if (s_skip) {                               // an earlier CTA gave up: drain the grid quickly
+    tc_fill_nan(p, b, hkv * R + 2 * pr, plan.nheads, s0);
+    return;
+  }
   const int64_t bhk = (int64_t)b * p.H_KV + hkv;
   const int64_t bhq0 = (int64_t)b * p.H_Q + hkv * R + 2 * pr;
   const int wla = p.W > 0 ? (max(0, s0 - (p.W - 1)) / 64) * 64 : s0;
@@ -246,6 +262,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap mQi, const __grid_constant
     for (int i = 0; i < kKStages; ++i) { mbar_init(k_full + i, 1); mbar_init(k_empty + i, plan.nheads); }
     for (int i = 0; i < kVStages; ++i) { mbar_init(v_full + i, 1); mbar_init(v_empty + i, plan.nheads); }
     for (int i = 0; i < 4; ++i) { mbar_init(s_full + i, 1); mbar_init(p_ready + i, 128); mbar_init(pv_done + i, 1); }
+    mbar_init(drained, 1); mbar_init(drained + 1, 1);
     *abort_flag = 0;
     fence_mbar_init();
   }
@@ -311,6 +328,12 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap mQi, const __grid_constant
         if (*abort_flag) break;
         if (++idle > 2000000u) { *abort_flag = 1; break; }
       }
+      // A block must not end with copies under way to its shared memory, also where it gives up: wait for the last load
+      // of every slot (a slot without one answers at once)
+      bool landed = mbar_wait_bounded(q_full, 0, kDrainPolls);
+      for (int i = 0; i < kKStages; ++i) landed = mbar_wait_bounded(k_full + i, i < ck.stage ? ck.par : ck.par ^ 1u, kDrainPolls) && landed;
+      for (int i = 0; i < kVStages; ++i) landed = mbar_wait_bounded(v_full + i, i < cv.stage ? cv.par : cv.par ^ 1u, kDrainPolls) && landed;
+      if (!landed) *abort_flag = 1;
     }
   } else if (warp >= 9) {
     // ------------------------------------------------------------ MMA issuers: warp 9 for head A, warp 10 for head B
@@ -433,6 +456,9 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap mQi, const __grid_constant
           if (more) { ++tq; cq.next(plan); }
         }
       }
+      // the same for products that write tensor memory
+      if (tc::elect_one()) tc::mma_commit(drained + h);
+      if (!__all_sync(0xffffffffu, mbar_wait_bounded(drained + h, 0, kDrainPolls))) *abort_flag = 1;
     }
   } else {
     // ------------------------------------------------------------ softmax: one thread per query row and head
@@ -687,7 +713,10 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap mQi, const __grid_constant
   }
   tc::fence_before_sync();
   __syncthreads();
-  if (tid == 0 && *abort_flag) atomicOr(p.status, 2);
+  if (*abort_flag) {
+    if (tid == 0) atomicOr(p.status, 2);
+    tc_fill_nan(p, b, hkv * R + 2 * pr, plan.nheads, s0);
+  }
   if (warp == 8) tc::tmem_dealloc(tmem_base, kTmemCols);
 }
 

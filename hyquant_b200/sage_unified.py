@@ -237,7 +237,9 @@ def hybrid_prefill(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, vertical_i
                    window_size: int, sm_scale: Optional[float], smooth_k: bool,
                    scale_granularity: Optional[str] = None, pv_fp8: bool = False) -> torch.Tensor:
     """Causal attention [B,H_q,N,D] with INT8 QK^T on the non-vertical prefix and BF16 on the
-    vertical lines and the window.  ``vertical_indices`` int64 [B,H_q,T] (any order) or None."""
+    vertical lines and the window.  ``vertical_indices`` int64 [B,H_q,T] (any order) or None.  Nothing is read back
+    from the device: should a bounded wait of the kernel ever run out, the rows it did not compute are NaN
+    (``PrefillPlan.check_status`` reads the status word)."""
     return PrefillPlan(q, k, v, vertical_indices, window_size, sm_scale, smooth_k, scale_granularity, pv_fp8, alias_inputs=True).run()
 
 

@@ -408,7 +408,7 @@ typedef struct hq_prefill_args {
   const void* vert_vt;
   const int32_t* nv_valid;
   void* out; int64_t o_sb, o_sh, o_sn;         /* [B,H_Q,N,128], strides in elements (multiples of 8) */
-  int32_t* status;             /* device word, zeroed by the caller; bit 1 = a bounded wait expired */
+  int32_t* status;             /* device word, zeroed by the caller; bit 1 = a bounded wait expired: rows not computed are NaN */
   /* FP8 P V (pv_fp8 != 0): P~ = 2^(s - m + 8.807) rounded to e4m3 against the exact running maximum,
    * V^T as e4m3 with one scale per channel (hq_prefill_quant_v_fp8), the product on tcgen05 kind::f8f6f4, the row sum
    * in fp32 before the cast - the arithmetic of the reference's sage_fp8_attention

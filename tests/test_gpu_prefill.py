@@ -176,6 +176,22 @@ def test_plan_reuse_and_status_word():
     check(a, orc.dense_causal_attention(q, k, v))
 
 
+@pytest.mark.parametrize("H_Q,H_KV,N,dtype,pv_fp8", [(4, 2, 300, torch.bfloat16, False), (3, 1, 129, torch.float32, True), (2, 2, 64, torch.float16, False)])
+def test_blocks_skipped_after_a_failed_wait_give_nan(H_Q, H_KV, N, dtype, pv_fp8):
+    """The status word as a block that gave up leaves it: the blocks that find it set skip their work; their rows must not
+    look like results.  The word cleared, the same plan computes."""
+    q, k, v = [t_bf16(x).to(dtype) for x in make(2, H_Q, H_KV, N, 64, N)]
+    plan = su.PrefillPlan(q, k, v, None, 64, None, True, pv_fp8=pv_fp8)
+    plan.out.fill_(7.0)
+    plan.status.fill_(2)
+    assert plan.run().isnan().all()
+    with pytest.raises(hq.HyQuantError):
+        plan.check_status()
+    plan.status.zero_()
+    assert plan.run().isfinite().all()
+    plan.check_status()
+
+
 def test_window_only_full_and_int8_only_variants():
     q, k, v = make(1, 8, 2, 700, 128, 5)
     ref = orc.dense_causal_attention(q, k, v)

@@ -477,17 +477,19 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap mQi, const __grid_constant
     bool ok = true;
     int ks_slot = 0;
     if constexpr (kFp8) {
-      // The scores of a tile.  tcgen05.ld is asynchronous: the next tile's are asked for as soon as this tile's registers
-      // are free (P is packed), so that the load runs under the store of P and the hand-over.
+      // The scores of tile t.  tcgen05.ld is asynchronous: its wait stands right behind it, because the compiler may copy
+      // registers wherever control flow meets and does not know that these are still being written.  (Asking for the
+      // next scores before the hand-over of P, with the wait in the next iteration, gave no such guarantee and was not
+      // faster either: 16K 2946 us, with load and wait around the hand-over 3208, like this 2936.)
       uint32_t sr[64];
-      auto load_scores = [&](int t) {
+      auto fetch = [&](int t) {
+        ok = __all_sync(0xffffffffu, tc::mbar_wait_abortable(s_full + 2 * h + (t & 1), (uint32_t)((t >> 1) & 1), abort_flag));
+        if (!ok) return;
         tc::fence_after_sync();
         tc::tmem_ld32(lane_base + colS + (t & 1) * 64, *reinterpret_cast<uint32_t(*)[32]>(&sr[0]));
         tc::tmem_ld32(lane_base + colS + (t & 1) * 64 + 32, *reinterpret_cast<uint32_t(*)[32]>(&sr[32]));
-      };
-      auto fetch = [&](int t) {        // wait for the scores of tile t and ask for them
-        ok = __all_sync(0xffffffffu, tc::mbar_wait_abortable(s_full + 2 * h + (t & 1), (uint32_t)((t >> 1) & 1), abort_flag));
-        if (ok) load_scores(t);
+        tc::tmem_wait_ld();
+        tc::tie64(sr);
       };
       auto tile = [&](int t, auto int8_tile) {
         constexpr bool kI8 = decltype(int8_tile)::value;
@@ -505,8 +507,6 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap mQi, const __grid_constant
           mlo = lim >= 31 ? 0u : lim < 0 ? 0xFFFFFFFFu : (0xFFFFFFFFu << (lim + 1));
           mhi = lim >= 63 ? 0u : lim < 32 ? 0xFFFFFFFFu : (0xFFFFFFFFu << (lim - 31));
         }
-        tc::tmem_wait_ld();
-        tc::tie64(sr);
         float* y = reinterpret_cast<float*>(sr);
         // scores before the row's factor `esc` (INT8: s32 -> fp32 by the magic-number add, key scale and bias in one
         // packed fma; BF16 tiles: masked columns -inf)
@@ -558,23 +558,19 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap mQi, const __grid_constant
 #pragma unroll
         for (int c = 0; c < 64; c += 4) pk[c >> 2] = tc::pack_e4m3x4(y[c], y[c + 1], y[c + 2], y[c + 3]);
         l += lsum;
-        // sr is free: if the next scores are there already, their load runs under the hand-over of P
-        const bool early = t + 1 < n_tiles &&
-                           __all_sync(0xffffffffu, mbar_test_wait(s_full + 2 * h + ((t + 1) & 1), (uint32_t)(((t + 1) >> 1) & 1)));
-        if (early) load_scores(t + 1);
         // P~ as e4m3 over the first 16 columns of the S buffer just read: row r in lane r, keys 4c .. 4c + 3 in column c
         tc::tmem_st16(tS, pk);
         tc::tmem_wait_st();
         tc::fence_before_sync();
         tc::mbar_arrive(p_ready + 2 * h + (t & 1));
-        if (!early && t + 1 < n_tiles) fetch(t + 1);
+        if (t + 1 < n_tiles) fetch(t + 1);
       };
       if (n_tiles > 0) fetch(0);
       int t = 0;
       for (; ok && t < n_rest && t < n_tiles; ++t) tile(t, TcTrue{});
       for (; ok && t < n_tiles; ++t) tile(t, TcFalse{});
     } else {
-      // (Asking for the next scores early, as above, was measured slower here: 9.37 against 9.25 ms at 32K.  So were two
+      // (Asking for the next scores before the hand-over of P was measured slower here: 9.37 against 9.25 ms at 32K.  So were two
       // threads per row, sixteen softmax warps in all: 10.1 ms - the loop lives on shared-memory bandwidth, of which
       // the key scales and biases of 256 rows take 1024 clocks of some 2200 per pair of tiles and the operands of
       // the products 640, and on the issuing warps' latency, which more warps lengthen.)

@@ -64,9 +64,9 @@ __global__ void kmean_final_kernel(const float* __restrict__ partial, int N, int
 // instruction, the sign put back on four packed bytes at a time.  Rounding half away from zero is |y| + 0.5 cut off, and
 // y has to be the correctly rounded quotient (a bf16 value over a 127th of another lies exactly on a tie often enough
 // that falling back near ties meant falling back in most warps): Markstein's division (IBM J. Res. Dev. 34, 1990),
-// the product with the rounded reciprocal corrected once by its exact remainder.  Rows whose maximum is infinite, NaN or
-// out of that method's range take the divide instruction element by element: x / inf = 0, inf / inf = NaN, which the
-// clamp turns into the lowest code.
+// the product with the rounded reciprocal corrected once by its exact remainder.  Rows that hold a
+// NaN, and rows whose maximum is infinite or out of that method's range, take the divide instruction element by element:
+// x / inf = 0; NaN (inf / inf too) becomes the lowest code in the clamp.
 __device__ __noinline__ void row_codes_exact(const float (&v)[16], float sc, uint32_t (&code)[4]) {
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -164,7 +164,7 @@ row_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t sb, int64_t sh, in
     const uint32_t flipped = n ^ neg;                                       // n <= 127: minus n is its complement plus one
     code[i] = ((flipped & 0x7F7F7F7Fu) + (neg & 0x01010101u)) ^ (flipped & 0x80808080u);
   }
-  if (!(amax >= 1e-25f && amax <= 1e30f)) {
+  if (top > 0x7F80u || !(amax >= 1e-25f && amax <= 1e30f)) {
     float v[16];                        // arrays of their own: what goes to the call by address must not be the common path's
     uint32_t exact[4];
 #pragma unroll

@@ -58,7 +58,7 @@ def test_operand_preparation_bit_exact(N, smooth):
 
 def test_row_codes_on_and_beside_ties():
     """Rows whose quotients are half-integers or one step beside them, all-zero rows, rows of the smallest values: the
-    codes of the division, bit for bit (the kernel multiplies by the reciprocal except near a tie)."""
+    codes of the division, bit for bit (the kernel corrects the product with the reciprocal by its remainder)."""
     rng = np.random.Generator(np.random.PCG64(3))
     N = 333
     k = (rng.integers(-127, 127, size=(1, 2, N, 128)) + 0.5).astype(np.float32)
@@ -76,6 +76,34 @@ def test_row_codes_on_and_beside_ties():
     assert np.array_equal(k_i8.cpu().numpy()[:, :, live], ki[:, :, live])
     assert np.array_equal(k_sc.cpu().numpy()[..., :N][..., live], ks[..., live])
     assert not k_i8.cpu().numpy()[:, :, 220:222].any()
+
+
+def test_row_codes_of_nan_and_infinite_elements():
+    """A NaN does not count for its row's maximum and gets the lowest code; its neighbours are quantised as without it.  In a
+    row with an infinity the finite elements are 0 and the infinity (inf / inf) is the lowest code."""
+    rng = np.random.Generator(np.random.PCG64(11))
+    N = 100
+    x = orc.bf16_round(rng.standard_normal((1, 2, N, 128), dtype=np.float32))
+    x[0, :, 3, 7] = np.nan
+    x[0, :, 40, [0, 31, 32, 127]] = np.nan
+    x[0, :, 41] = np.nan
+    x[0, :, 63, 5] = np.inf
+    x[0, :, 64, 90] = -np.inf
+    x[0, :, 65, 1], x[0, :, 65, 2] = np.inf, np.nan
+    sm = 1.0 / orc.LOG2E                                     # q is scaled by sm * log2 e = 1, up to the fp32 rounding
+    q_i8, _, q_sc, k_i8, _, k_sc, _ = su.quantize_operands(t_bf16(x), t_bf16(x), sm, False)
+    with np.errstate(invalid="ignore"):
+        amax = np.fmax.reduce(np.abs(x), axis=-1, initial=0.0)
+        scale = (np.maximum(amax, np.float32(1e-30)) / np.float32(127.0)).astype(np.float32)
+        y = (x / scale[..., None]).astype(np.float32)
+        y = np.trunc(y + np.where(y >= 0, np.float32(0.5), np.float32(-0.5)))
+    codes = np.where(np.isnan(y), -128, np.clip(np.nan_to_num(y), -128, 127)).astype(np.int8)
+    assert np.array_equal(k_i8.cpu().numpy(), codes)
+    assert np.array_equal(k_sc.cpu().numpy()[..., :N], scale)
+    special = [3, 40, 41, 63, 64, 65]
+    low = np.isnan(y[:, :, special])
+    assert (q_i8.cpu().numpy()[:, :, special][low] == -128).all()
+    assert (np.abs(q_i8.cpu().numpy().astype(int) - codes.astype(int)) <= 1).all()
 
 
 @pytest.mark.parametrize("T,last", [(1, 0), (64, 63), (65, 4000), (1600, 32639), (500, 100), (16384, (1 << 20) - 1)])

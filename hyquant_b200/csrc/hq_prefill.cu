@@ -55,37 +55,19 @@ vertical_meta_kernel(const int* __restrict__ vasc, int T, int N, int Npad, int W
 }
 
 // idx int64 [rows, T] in any order -> asc int32 [rows, T]: clamped to [0, last], ascending (a position given twice
-// stays twice).  Latency-bound, one CTA per row: a bitmap of the positions in shared memory, a scan over its words'
-// counts, and each thread writes the positions of its words out in order; what the bitmap already held when it was
-// set (a repeated position) goes to a side list, and every entry then moves up by the number of side entries below it.
+// stays twice).  Latency-bound, one CTA per row: a bitmap of the positions in shared memory and a scan over its words'
+// counts; each thread then writes the positions of its words out in order.  Where a position is repeated (the clamp
+// makes that of lists with positions out of range), the entries are counted per distinct position instead, and every
+// entry takes the next place of its position: linear in T however often one is repeated (moving each position up by a
+// walk over a side list of the repeated entries was quadratic: milliseconds for 16384 entries over 100 positions).
 // Takes the place of a clamp, a library sort with its index arrays and two conversions (40 us for 32 rows x 400).
 constexpr int kSortThreads = 1024;
 constexpr int kSortMaxT = 16384, kSortMaxLast = 1 << 20;
-__global__ void __launch_bounds__(kSortThreads)
-vertical_sort_kernel(const int64_t* __restrict__ idx, int T, int last, int32_t* __restrict__ asc) {
-  extern __shared__ uint32_t s_bits[];                     // [words], then the side list [T]
-  const int words = last / 32 + 1;
-  int* extra = reinterpret_cast<int*>(s_bits + words);
-  __shared__ int s_extra;
-  __shared__ int warp_sums[32];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int64_t* src = idx + (int64_t)blockIdx.x * T;
-  int32_t* dst = asc + (int64_t)blockIdx.x * T;
-  for (int i = tid; i < words; i += kSortThreads) s_bits[i] = 0u;
-  if (tid == 0) s_extra = 0;
-  __syncthreads();
-#pragma unroll 4
-  for (int i = tid; i < T; i += kSortThreads) {
-    const int64_t raw = __ldg(src + i);
-    const int v = raw < 0 ? 0 : raw > last ? last : (int)raw;
-    const uint32_t bit = 1u << (v & 31);
-    if (atomicOr(&s_bits[v >> 5], bit) & bit) extra[atomicAdd(&s_extra, 1)] = v;
-  }
-  __syncthreads();
-  const int per = (words + kSortThreads - 1) / kSortThreads, w0 = min(words, tid * per), w1 = min(words, w0 + per);
-  int count = 0;
-  for (int w = w0; w < w1; ++w) count += __popc(s_bits[w]);
-  int inc = count;
+
+// exclusive prefix of v over the block's 1024 threads
+__device__ __forceinline__ int sort_block_scan(int v, int* warp_sums) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int inc = v;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
     const int n = __shfl_up_sync(0xffffffffu, inc, o);
@@ -104,16 +86,62 @@ vertical_sort_kernel(const int64_t* __restrict__ idx, int T, int last, int32_t* 
     warp_sums[lane] = ws - own;
   }
   __syncthreads();
-  const int ne = s_extra;
-  int pos = warp_sums[warp] + inc - count;
-  for (int w = w0; w < w1; ++w) {
-    for (uint32_t m = s_bits[w]; m != 0u; m &= m - 1u) {
-      const int v = w * 32 + __ffs(m) - 1;
-      int below = 0, equal = 0;
-      for (int e = 0; e < ne; ++e) { below += extra[e] < v; equal += extra[e] == v; }
-      for (int j = 0; j <= equal; ++j) dst[pos + below + j] = v;
-      ++pos;
-    }
+  return warp_sums[warp] + inc - v;
+}
+
+__global__ void __launch_bounds__(kSortThreads)
+vertical_sort_kernel(const int64_t* __restrict__ idx, int T, int last, int32_t* __restrict__ asc) {
+  extern __shared__ uint32_t s_bits[];                     // [words], then an entry count per distinct position [T]
+  const int words = last / 32 + 1;
+  int* places = reinterpret_cast<int*>(s_bits + words);
+  __shared__ int first_rank[kSortThreads];                 // distinct positions below each thread's words
+  __shared__ int warp_sums[32];
+  const int tid = threadIdx.x;
+  const int64_t* src = idx + (int64_t)blockIdx.x * T;
+  int32_t* dst = asc + (int64_t)blockIdx.x * T;
+  auto position = [&](int i) {
+    const int64_t raw = __ldg(src + i);
+    return raw < 0 ? 0 : raw > last ? last : (int)raw;
+  };
+  for (int i = tid; i < words; i += kSortThreads) s_bits[i] = 0u;
+  __syncthreads();
+  int repeated = 0;
+#pragma unroll 4
+  for (int i = tid; i < T; i += kSortThreads) {
+    const int v = position(i);
+    const uint32_t bit = 1u << (v & 31);
+    repeated |= (atomicOr(&s_bits[v >> 5], bit) & bit) != 0u;
+  }
+  repeated = __syncthreads_or(repeated);
+  const int per = (words + kSortThreads - 1) / kSortThreads, w0 = min(words, tid * per), w1 = min(words, w0 + per);
+  int count = 0;
+  for (int w = w0; w < w1; ++w) count += __popc(s_bits[w]);
+  int pos = sort_block_scan(count, warp_sums);
+  if (!repeated) {
+    for (int w = w0; w < w1; ++w)
+      for (uint32_t m = s_bits[w]; m != 0u; m &= m - 1u) dst[pos++] = w * 32 + __ffs(m) - 1;
+    return;
+  }
+  first_rank[tid] = pos;
+  for (int i = tid; i < T; i += kSortThreads) places[i] = 0;
+  __syncthreads();
+  auto rank = [&](int v) {                                 // distinct positions below v
+    const int word = v >> 5, owner = word / per;
+    int r = first_rank[owner] + __popc(s_bits[word] & ((1u << (v & 31)) - 1u));
+    for (int w = owner * per; w < word; ++w) r += __popc(s_bits[w]);
+    return r;
+  };
+  for (int i = tid; i < T; i += kSortThreads) atomicAdd(&places[rank(position(i))], 1);
+  __syncthreads();
+  const int tper = (T + kSortThreads - 1) / kSortThreads, t0 = min(T, tid * tper), t1 = min(T, t0 + tper);
+  int entries = 0;
+  for (int i = t0; i < t1; ++i) entries += places[i];
+  int base = sort_block_scan(entries, warp_sums);
+  for (int i = t0; i < t1; ++i) { const int n = places[i]; places[i] = base; base += n; }
+  __syncthreads();
+  for (int i = tid; i < T; i += kSortThreads) {
+    const int v = position(i);
+    dst[atomicAdd(&places[rank(v)], 1)] = v;               // equal entries: any order is the same list
   }
 }
 

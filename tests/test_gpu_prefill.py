@@ -119,6 +119,36 @@ def test_vertical_sort_is_the_clamped_ascending_list(T, last):
     assert torch.equal(asc.long(), idx.clamp(0, last).sort(dim=-1).values)
 
 
+@pytest.mark.parametrize("T,last", [(16384, 99), (16384, (1 << 20) - 1), (5000, 40000)])
+def test_vertical_sort_of_lists_that_repeat_positions_is_linear(T, last):
+    """Long lists over few positions, every position twice, one position in half of the places: the sorted list, in not
+    much more time than a list without repetitions takes (each form is one launch of a few passes; a walk over the
+    repeated entries per position took over a hundred times as long)."""
+    g = torch.Generator(device=DEV); g.manual_seed(T)
+    lib, asc = hq._lib.lib(), torch.empty(1, T, dtype=torch.int32, device=DEV)
+
+    def run(idx, last):
+        assert lib.hq_prefill_vertical_sort(idx.data_ptr(), 1, T, last, asc.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+
+    def best_us(idx, last):
+        times = []
+        for _ in range(8):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record(); run(idx, last); b.record(); b.synchronize()
+            times.append(a.elapsed_time(b) * 1e3)
+        return min(times)
+
+    plain = torch.randperm(1 << 20, generator=g, device=DEV)[None, :T].contiguous()
+    limit = 12 * best_us(plain, (1 << 20) - 1)
+    some = torch.randint(0, last + 1, (1, T), generator=g, device=DEV)
+    twice = some.clone(); twice[:, 1::2] = some[:, ::2][:, :T // 2]
+    half = some.clone(); half[:, ::2] = last // 3
+    for idx in (some % 100, twice, half, torch.full_like(some, last)):
+        run(idx, last)
+        assert torch.equal(asc.long(), idx.clamp(0, last).sort(dim=-1).values)
+        assert best_us(idx, last) <= limit
+
+
 def test_the_one_shot_calls_leave_their_inputs_alone():
     """The one-shot entry points may read q and k in place where a plan copies them: same result, inputs unchanged."""
     q, k, v = make(2, 4, 2, 333, 128, 3)

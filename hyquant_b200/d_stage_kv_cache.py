@@ -315,6 +315,8 @@ class DStageLayerCache:
         if out is None:
             out = torch.empty_like(query_states, memory_format=torch.contiguous_format)
         stream = _lib.stream_ptr(p.device)
+        if stream != p.stream:
+            p.follow_stream(stream)
         if key_states is not None:
             a.k_new, a.v_new, a.kn_stride, a.vn_stride = k_ptr, v_ptr, 128, 128
         a.n_quant, a.n_staging = self._n_quant, self._staging_ptr
@@ -444,19 +446,17 @@ class DStageLayerCache:
         k2, v2 = key_states.reshape(B * H_KV, D), value_states.reshape(B * H_KV, D)
         plan = self._decode_plan(q2d, kv_repeat)
         a = plan.args
-        own = (a.num_splits, a.workspace, a.workspace_bytes, a.flags)
+        own = (a.num_splits, a.flags)
         a.flags = _lib.HQ_DECODE_OVERLAP_PREVIOUS if (overlap and self.k_bits == 4 and self.v_bits == 4) else 0
         a.k_new, a.v_new, a.kn_stride, a.vn_stride = k2.data_ptr(), v2.data_ptr(), k2.stride(0), v2.stride(0)
         a.num_splits = num_splits
         if num_splits > 0:
             a.flags |= _lib.HQ_DECODE_SHARED_CHIP
-        if workspace is not None:
-            a.workspace, a.workspace_bytes = workspace.data_ptr(), workspace.numel()
         try:
-            plan.run(q2d, out=out.view(B_ * H_Q_, D_))
+            plan.run(q2d, out=out.view(B_ * H_Q_, D_), workspace=workspace)
         finally:
             a.k_new = a.v_new = None
-            a.num_splits, a.workspace, a.workspace_bytes, a.flags = own
+            a.num_splits, a.flags = own
 
     def count_replayed_step(self):
         """Account for one replay of a launch captured by :meth:`capture_decode_step` (one token appended)."""

@@ -222,6 +222,7 @@ class DecodePlan:
                 a.n_staging, a.k_staging, a.v_staging, a.kg_stride_bh, a.vg_stride_bh = n, kptr, vptr, kst, vst
             else:
                 a.n_window, a.k_window, a.v_window, a.kw_stride_bh, a.vw_stride_bh = n, kptr, vptr, kst, vst
+        self.stream = _lib.stream_ptr(q.device)
         self.ws = decode_workspace(q.device, self.BH_KV, kv_repeat)
         a.workspace, a.workspace_bytes = self.ws.data_ptr(), self.ws.numel()
         self.args = a
@@ -229,9 +230,21 @@ class DecodePlan:
         self._keep = keep
         self._fn = _lib.lib().hq_decode_splitk
 
-    def run(self, q: torch.Tensor, out: Optional[torch.Tensor] = None, partial=None, peer=None) -> torch.Tensor:
+    def follow_stream(self, stream: int) -> None:
+        """Point the arguments at the workspace of ``stream``, the current one, if the plan was last used on another: plans
+        of one shape share a workspace per stream, and two launches that run at the same time must not share one.  A
+        launch that is being captured keeps the plan's workspace (nothing is allocated under capture); replays then have
+        to be ordered with the plan's other launches by whoever replays them."""
+        if stream != self.stream and not torch.cuda.is_current_stream_capturing():
+            self.ws = decode_workspace(self.device, self.BH_KV, self.kv_repeat)
+            self.args.workspace, self.args.workspace_bytes = self.ws.data_ptr(), self.ws.numel()
+            self.stream = stream
+
+    def run(self, q: torch.Tensor, out: Optional[torch.Tensor] = None, partial=None, peer=None,
+            workspace: Optional[torch.Tensor] = None) -> torch.Tensor:
         """Launch on the current stream.  ``partial=(m, l, acc)`` fp32 tensors
-        selects the un-normalised (sequence-sharded) output.  ``peer=(exchange, seq)``
+        selects the un-normalised (sequence-sharded) output.  ``workspace``: split-K scratch for this launch instead of
+        the stream's.  ``peer=(exchange, seq)``
         (a ``sharded.PeerExchange`` and the call's sequence number): this call covers one
         sequence shard; the kernel exchanges its state with the other ranks and ``out`` is
         the merged result."""
@@ -252,7 +265,15 @@ class DecodePlan:
                 out = torch.empty(q.shape[0], 128, dtype=q.dtype, device=q.device)
             a.partial_m = a.partial_l = a.partial_acc = None
             a.out, a.out_stride, a.out_dtype = out.data_ptr(), out.stride(0), _lib.dtype_code(out.dtype)
-        rc = self._fn(C.byref(a), _lib.stream_ptr(self.device))
+        stream = _lib.stream_ptr(self.device)
+        if workspace is None:
+            self.follow_stream(stream)
+            rc = self._fn(C.byref(a), stream)
+        else:
+            own = a.workspace, a.workspace_bytes
+            a.workspace, a.workspace_bytes = workspace.data_ptr(), workspace.numel()
+            rc = self._fn(C.byref(a), stream)
+            a.workspace, a.workspace_bytes = own
         if rc != 0:
             _lib.check(rc, "hq_decode_splitk")
         return out

@@ -39,6 +39,7 @@
 // workspace with an atomic ticket: the last CTA of a head does the
 // log-sum-exp merge and writes the output, so there is no second launch.
 #include "hq_decode_kernel.cuh"
+#include "hq_kept.h"
 
 namespace hq {
 
@@ -48,16 +49,10 @@ namespace hq {
 // the box), units per plane, planes}, box {unit, 1, 2}, no swizzle.  Maps are kept by what they are made of (a
 // cache's buffers change only when it grows), since encoding one costs about as much host time as the launch.
 static int kv_tensor_map(CUtensorMap* out, const void* base, int row_bytes, int64_t plane_tokens, int64_t planes, int unit_tokens) {
-  struct Entry { const void* base; int row; int64_t tokens, planes; int unit; CUtensorMap map; };
-  // one place per cache of a model's layers: with eight places in turn a model of 32 layers encoded a map on every call
-  constexpr int kKeep = 128;
-  static thread_local Entry kept[kKeep];
-  const uint64_t mixed = (uint64_t)(uintptr_t)base * 0x9E3779B97F4A7C15ull;
-  Entry& e = kept[mixed >> 57];
-  if (e.base == base && e.row == row_bytes && e.tokens == plane_tokens && e.planes == planes && e.unit == unit_tokens) {
-    *out = e.map;
-    return HQ_OK;
-  }
+  static thread_local Kept<PlanesKey, CUtensorMap> kept;
+  PlanesKey key;
+  key.base = base; key.tokens = plane_tokens; key.planes = planes; key.row = row_bytes; key.unit = unit_tokens;
+  if (const CUtensorMap* m = kept.find(key)) { *out = *m; return HQ_OK; }
   tc::EncodeTiledFn fn = tc::encode_fn();
   HQ_REQUIRE(fn != nullptr, HQ_ERR_CUDA, "hq_decode_splitk: cuTensorMapEncodeTiled is not available from this driver");
   const cuuint64_t unit_bytes = (cuuint64_t)row_bytes * (cuuint64_t)unit_tokens;
@@ -70,7 +65,7 @@ static int kv_tensor_map(CUtensorMap* out, const void* base, int row_bytes, int6
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   HQ_REQUIRE(r == CUDA_SUCCESS, HQ_ERR_CUDA, "hq_decode_splitk: cuTensorMapEncodeTiled failed with %d (row %d, %lld tokens, %lld planes)",
              (int)r, row_bytes, (long long)plane_tokens, (long long)planes);
-  e = Entry{base, row_bytes, plane_tokens, planes, unit_tokens, *out};
+  kept.keep(key, *out);
   return HQ_OK;
 }
 

@@ -49,6 +49,7 @@ class DecodeStepGraph:
             layer.bind_lengths(self._len[i])
         self._graph = None
         self._ws, self._streams = [], []         # one split-K workspace per branch of the graph, and the branches' streams
+        self._used_on = {_lib.stream_ptr(self.dev_in.device)}    # streams the device buffers are safe to be freed behind
         self._warm = False
 
     BRANCHES = 16
@@ -90,6 +91,7 @@ class DecodeStepGraph:
             _lib.check(_lib.lib().hq_decode_workspace_bytes(self.B * self.H_KV, self.R, C.byref(nbytes)), "hq_decode_workspace_bytes")
             self._ws = [torch.zeros(int(nbytes.value), dtype=torch.uint8, device=dev) for _ in range(branches)]
             self._streams = [torch.cuda.Stream(dev) for _ in range(branches - 1)]
+            self._used_on = set()
         with torch.cuda.graph(g):
             main = torch.cuda.current_stream(dev)
             self.dev_in.copy_(self.host_in, non_blocking=True)
@@ -105,6 +107,16 @@ class DecodeStepGraph:
             self.host_out.copy_(self.dev_out, non_blocking=True)
         self._graph = g
         self._ptrs = [l._kq.data_ptr() for l in self.layers]
+
+    def _follow_stream(self):
+        """A replay may run on another stream than the one the buffers were allocated on, and it need not be over when
+        :meth:`close` or the end of this object gives them back: the allocator has to know of that stream."""
+        stream = _lib.stream_ptr(self.dev_in.device)
+        if stream not in self._used_on:
+            current = torch.cuda.current_stream(self.dev_in.device)
+            for t in (self.dev_in, self.dev_out, *self._ws):
+                t.record_stream(current)
+            self._used_on.add(stream)
 
     def step(self, synchronize: bool = True) -> torch.Tensor:
         """Run one token: ``host_q / host_k / host_v`` hold the new rows of every layer; returns ``host_out``
@@ -126,6 +138,7 @@ class DecodeStepGraph:
         else:
             if self._graph is None:
                 self._capture()
+            self._follow_stream()
             self._graph.replay()
             for layer in self.layers:
                 layer.count_replayed_step()

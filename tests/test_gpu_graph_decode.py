@@ -85,6 +85,31 @@ def test_layers_on_branches_equal_layer_by_layer(n, B, H_Q, H_KV, N, W):
     g.close()
 
 
+def test_buffers_are_not_given_back_before_a_replay_on_another_stream_ends(monkeypatch):
+    """close() right behind an asynchronous replay on a side stream: every device buffer of the graph, the branches'
+    workspaces among them, is registered with the allocator for that stream (once)."""
+    B, H_Q, H_KV = 1, 4, 2
+    layers = _layers(3, B, H_Q, H_KV, 300, 64)
+    g = DecodeStepGraph(layers, B, H_Q, H_KV)
+    for t in (*g.host_q, *g.host_k, *g.host_v):
+        t.normal_()
+    g.step()
+    first = g.step().clone()
+    seen, real = [], torch.Tensor.record_stream
+    monkeypatch.setattr(torch.Tensor, "record_stream", lambda t, st: (seen.append((t.data_ptr(), st.cuda_stream)), real(t, st))[1])
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        g.step(synchronize=False)
+        g.step(synchronize=False)
+        want = {(t.data_ptr(), side.cuda_stream) for t in (g.dev_in, g.dev_out, *g._ws)}
+        assert len(g._ws) == 3 and set(seen) == want and len(seen) == len(want)
+        out = g.host_out
+        g.close()
+    torch.cuda.synchronize()
+    assert out.float().isfinite().all() and first.shape == out.shape
+
+
 def test_lengths_record_overrides_the_arguments():
     """The kernel must follow the device record, not the launch arguments."""
     (layer,) = _layers(1, 1, 8, 2, 900, 64)

@@ -88,14 +88,19 @@ def per_block_int8(q: torch.Tensor, k: torch.Tensor, km: Optional[torch.Tensor] 
     return qi, qs, ki, ks
 
 
+def _granularity(scale_granularity: Optional[str]) -> str:
+    gran = SCALE_GRANULARITY if scale_granularity is None else scale_granularity
+    if gran not in ("row", "block"):
+        raise ValueError(f"scale_granularity must be 'row' or 'block', got {gran!r}")
+    return gran
+
+
 def quantize_operands(qb: torch.Tensor, kb: torch.Tensor, sm_scale: float, smooth_k: bool,
                       scale_granularity: Optional[str] = None, alias_q: bool = False):
     """Operand preparation (``hq_prefill_quant`` / ``hq_prefill_quant_blocks``): returns q_i8, q_bf, q_scale, k_i8,
     k_bf, k_scale, k_mean; the scale arrays hold one value per row either way.  ``alias_q``: q_bf may be ``qb`` itself
     (the BF16 query operand is the query row by row, so a contiguous query needs no copy)."""
-    gran = SCALE_GRANULARITY if scale_granularity is None else scale_granularity
-    if gran not in ("row", "block"):
-        raise ValueError(f"scale_granularity must be 'row' or 'block', got {gran!r}")
+    gran = _granularity(scale_granularity)
     B, H_q, N, _ = qb.shape
     H_kv = kb.shape[1]
     dev = qb.device
@@ -142,6 +147,7 @@ class PrefillPlan:
         st = _lib.stream_ptr(dev)
         if sm_scale is None:
             sm_scale = 128 ** -0.5
+        _granularity(scale_granularity)          # refused where nothing is quantised, too
         nqb, nkb = (N + 127) // 128, (N + 63) // 64
         # A window that covers the prompt leaves no INT8 tile and no vertical line (16-bit causal attention): without K
         # smoothing the BF16 operands are then q and k as they are, and nothing reads codes, scales or biases

@@ -182,6 +182,13 @@ def test_vertical_attention_vs_dense(B, H_Q, H_KV, N, W):
         assert max_abs(to_np(out), rr) <= MAX_ABS
 
 
+@pytest.mark.parametrize("window,smooth", [(64, True), (200, False), (500, False)])
+def test_an_unknown_scale_granularity_is_refused(window, smooth):
+    q, k, v = [t_bf16(x) for x in make(1, 2, 1, 200, 64, 4)]
+    with pytest.raises(ValueError):
+        su.hybrid_prefill(q, k, v, None, window, None, smooth, scale_granularity="tile")
+
+
 def uneven_lists(B, H_Q, N, W, T):
     """[B, H_Q, T] positions: heads in turn with all lines early, all late, spread, in the middle - every block then serves
     two heads with up to T / 64 tiles more for the one than for the other."""

@@ -160,6 +160,31 @@ def test_the_one_shot_calls_leave_their_inputs_alone():
         assert np.array_equal(to_np(tq), q) and np.array_equal(to_np(tk), k) and np.array_equal(to_np(tv), v)
 
 
+@pytest.mark.parametrize("form", ["tokens_first", "padded_rows", "every_other_head"])
+def test_the_one_shot_calls_on_strided_inputs(form):
+    """q, k and v as the models hand them over (transposed projections), as slices of wider rows and of more heads: the
+    results of contiguous tensors, bit for bit, on the hybrid, the 16-bit and the FP8 route; inputs unchanged."""
+    def strided(x):
+        t = t_bf16(x)
+        if form == "tokens_first":
+            return t.transpose(1, 2).contiguous().transpose(1, 2)
+        if form == "padded_rows":
+            return torch.cat([t, torch.full_like(t[..., :8], 3.0)], dim=-1)[..., :128]
+        return torch.stack([t, torch.full_like(t, 5.0)], dim=2).flatten(1, 2)[:, ::2]
+
+    N, W = 333, 64
+    q, k, v = make(2, 4, 2, N, W, 12)
+    a, b = [t_bf16(x) for x in (q, k, v)], [strided(x) for x in (q, k, v)]
+    assert all(torch.equal(x, y) and not y.is_contiguous() for x, y in zip(a, b))
+    idx = uneven_lists(2, 4, N, W, 40)
+    for call in (lambda t: su.hybrid_prefill(*t, idx, W, None, True), lambda t: su.hybrid_prefill(*t, None, N, None, False),
+                 lambda t: su.full_attention_fp16_triton(*t), lambda t: su.sage_fp8_attention(*t),
+                 lambda t: su.sage_unified_attention(*t, window_size=W, smooth_k=False)):
+        assert torch.equal(call(a), call(b))
+    for x, y in zip((q, k, v), b):
+        assert np.array_equal(to_np(y), x)
+
+
 def check(out, ref):
     assert np.isfinite(out).all()
     assert max_abs(out, ref) <= MAX_ABS, max_abs(out, ref)

@@ -111,6 +111,16 @@ def test_pooled_query_is_the_sum_in_token_order(tail, R, offset):
     k = torch.eye(128, device=DEV, dtype=torch.bfloat16).expand(1, 2, 128, 128).contiguous()
     keys = torch.cat([k, torch.zeros(1, 2, tail, 128, device=DEV, dtype=torch.bfloat16)], dim=2)
     got = hq.vertical_scores(q, keys, tail, 1, group_mean=R)
+    # the pooled query itself, from the buffer that the scoring call fills
+    lib, st = hq._lib.lib(), torch.cuda.current_stream().cuda_stream
+    pooled, scores = torch.empty(1, 2, 128, device=DEV), torch.empty(1, 2, 128, device=DEV)
+    rows = (q.data_ptr(), hq._lib.HQ_BF16, *q.stride()[:3], 1)
+    keys_of = (keys.data_ptr(), *keys.stride()[:3])
+    if R > 1:
+        rc = lib.hq_vertical_scores_grouped(*rows, 2, R, tail, tail, *keys_of, 128, 0, 0, pooled.data_ptr(), scores.data_ptr(), st)
+    else:
+        rc = lib.hq_vertical_scores(*rows, 2, tail, tail, *keys_of, 2, 128, 0, 0, pooled.data_ptr(), scores.data_ptr(), st)
+    assert rc == 0 and torch.equal(scores, got)
     m = q.float().reshape(1, 2, R, tail, 128).cpu().numpy()
     s = np.zeros((1, 2, tail, 128), np.float32)
     for r in range(R):
@@ -121,6 +131,7 @@ def test_pooled_query_is_the_sum_in_token_order(tail, R, offset):
     for i in range(tail):
         acc += s[:, :, i]
     want = acc / np.float32(tail)
+    assert np.array_equal(pooled.cpu().numpy(), want)
     # the scores split the mean into two bf16 parts: 2^-16 of the value at most
     assert np.all(np.abs(got.cpu().numpy() - want) <= 2.0 ** -16 * np.abs(want))
 

@@ -723,8 +723,8 @@ decode_splitk_kernel(const __grid_constant__ CUtensorMap kv_map, const DecodePar
       // scores of both 16-token chunks: this lane holds tokens g, g+8, 16+g, 24+g.  The loop is bound by instruction issue
       // and dependent latencies (two-tile form: 800 instructions a unit at 0.43 a clock and scheduler), so: the
       // accumulators start at minus the head's constant of the biased codes instead of losing it afterwards, only a
-      // head's last unit masks tokens, and the softmax works on pairs of heads (two-tile 128K x 4: 53.7 -> 52.5 us a call,
-      // batch 16 at 32K: 138.3 -> 137.1 us).
+      // head's last unit masks tokens, and the softmax works on pairs of heads (two-tile 128K x 4: 53.8 -> 52.6 us a call;
+      // the one-tile form at 32K and at batch 16 no faster by more than its runs differ).
       float s[kChunks][NT][4];
 #pragma unroll
       for (int ch = 0; ch < kChunks; ++ch)

@@ -59,7 +59,7 @@ vertical_meta_kernel(const int* __restrict__ vasc, int T, int N, int Npad, int W
 // counts; each thread then writes the positions of its words out in order.  Where a position is repeated (the clamp
 // makes that of lists with positions out of range), the entries are counted per distinct position instead, and every
 // entry takes the next place of its position: linear in T however often one is repeated (moving each position up by a
-// walk over a side list of the repeated entries was quadratic: milliseconds for 16384 entries over 100 positions).
+// walk over a side list of the repeated entries was quadratic: 16384 entries over 100 positions 4225 us, now 38; distinct ones 44 and 45).
 // Takes the place of a clamp, a library sort with its index arrays and two conversions (40 us for 32 rows x 400).
 constexpr int kSortThreads = 1024;
 constexpr int kSortMaxT = 16384, kSortMaxLast = 1 << 20;

@@ -9,8 +9,8 @@
 // interleave on the SM: while one head's threads are in their exponentials the tensor core runs the other
 // head's products.  11 warps:
 //   warp 8 (one lane)  producer: TMA tensor-map loads (128-byte swizzle) of both heads' Q once, then K tiles
-//                      and transposed V tiles into two four-slot rings (a K slot is free again after the
-//                      heads' Q K^T, a V slot after their P V).  INT8 and window items serve both heads;
+//                      and transposed V tiles into two rings of three and four slots (a K slot is free again
+//                      after the heads' Q K^T, a V slot after their P V).  INT8 and window items serve both heads;
 //                      the gathered vertical-line tiles are per head.
 //   warps 9, 10        (an elected lane each) issue tcgen05.mma for head A / B: S = Q K^T (kind::i8 with s32
 //                      accumulators, or kind::f16 on bf16) into one of the head's two S buffers in tensor
@@ -68,8 +68,8 @@ struct TcPlan {
   __device__ __forceinline__ int n_items() const { return n_rest + nvert0 + nvert1 + n_win; }
 };
 
-// The ring items of a CTA in load order, walked with counters only (the threads that walk it are single
-// lanes whose instruction latency paces the pipeline): the INT8 tiles, then the vertical-line tiles of the
+// The ring items of a CTA in load order, walked with counters only (one producer lane and the two converged issuing
+// warps walk it, and their instruction latency paces the pipeline): the INT8 tiles, then the vertical-line tiles of the
 // two heads interleaved (A's j-th, B's j-th, ...), then the window tiles.  INT8 and window items feed both
 // heads, a vertical item only its own head.
 struct TcItemIter {
@@ -93,7 +93,7 @@ struct TcItemIter {
   }
   __device__ __forceinline__ void next(const TcPlan& pl) {
     if (++stage == depth) { stage = 0; par ^= 1u; }
-    // the common cases first (the lanes that walk the ring are single threads: every instruction here is latency)
+    // the common cases first (a ring is walked by one lane or one warp: every instruction here is latency)
     if (kind == 0 && j + 1 < pl.n_rest) { ++j; return; }
     if (kind == 2) { if (++j >= pl.n_win) kind = 3; return; }
     do step(pl); while (kind < 3 && !valid(pl));

@@ -5,7 +5,10 @@ The reference appends and attends layer by layer from Python, with the cache len
 host message (every layer's new q / k / v rows), :class:`DecodeStepGraph` adds every layer's ``(n_quant, n_staging)``,
 and the replayed graph is copy in -> one fused append + attention launch per layer, side by side -> copy out.  The decode kernels
 read the lengths from the message (``hq_decode_args.lengths``), so the same graph serves every step; only the step on
-which a staging buffer fills (one in 128) runs eagerly, because it quantises 128 tokens first.
+which a staging buffer fills (one in 128) runs eagerly, because it quantises 128 tokens first, and so does the first.
+
+Every layer's rows have to be known before the step.  The layer-by-layer loop of one decoder, where the query of a layer
+is made from the output of the one before, calls :meth:`DStageLayerCache.decode_step` per layer instead.
 """
 
 from __future__ import annotations
@@ -60,9 +63,9 @@ class DecodeStepGraph:
         The launches share the chip, so they run as half-size blocks, two to an SM (HQ_DECODE_SHARED_CHIP).  Splits: as many
         as give sixteen launches in flight about 1.75 blocks per place (some wait and take over where others end), or, with
         few layers, one block per place; and no more than leave a warp four units (32 quantised or 8 BF16 tokens) to
-        work on.  Measured on 8 kv-heads: 32 layers of an 8K prefix 126 us with 4 splits (16 branches of full-size
-        blocks 143 to 165, one launch after the other 345), 16 layers of 16K 111 with 4 (115), 32 layers of 1K 75 with 2 to 4
-        (82), 8 layers of 2K 43 with 2 to 4 (48)."""
+        work on.  Measured on 8 kv-heads, the replay alone: 32 layers of an 8K prefix 126 us with 4 splits (16 branches of
+        full-size blocks 143 to 165), 16 layers of 16K 111 with 4 (115), 32 layers of 1K 75 with 2 to 4 (82), 8 layers of
+        2K 43 with 2 to 4 (48).  A whole step() of 32 layers of 8K: 148, with one launch after the other 346."""
         branches = min(self.BRANCHES, len(self.layers))
         if branches == 1:
             return 0, 1

@@ -60,6 +60,28 @@ struct TcSmem {              // offsets from a 1024-aligned base
   static constexpr int Total = Bar + 256;
 };
 
+// A converged warp's wait.  The first poll (which the hardware holds for a while) is inline and nearly always enough; the
+// poll loop is out of line, so that a wait is straight-line code.  A poll takes 40 clocks, but with the poll loop inline a
+// wait for a barrier that had long flipped took 300 to 450 in these loops: softmax and issuing warps fetch different
+// code through one instruction cache, and every taken branch of a wait, of the ring walk and of the two kinds of tiles went
+// somewhere cold.  With the waits straight, the INT8 tiles in loops of their own (softmax and issuing warps), and the three
+// waits of an issuing warp asked together: hybrid 8K 708 -> 667 us, 32K 9.01 -> 8.53 ms, FP8 16K 2.93 -> 2.81 ms, 16-bit
+// 2 x 1973 112 -> 107 us per call.
+static __device__ __noinline__ bool mbar_wait_rest(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+  return (bool)__all_sync(0xffffffffu, tc::mbar_wait_abortable(bar, parity, abort_flag));
+}
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+  if (__builtin_expect(__all_sync(0xffffffffu, mbar_try_wait(bar, parity)), 1)) return true;
+  return mbar_wait_rest(bar, parity, abort_flag);
+}
+// three at once: one vote where all are there
+__device__ __forceinline__ bool mbar_wait_warp3(uint64_t* b0, uint32_t p0, uint64_t* b1, uint32_t p1, uint64_t* b2, uint32_t p2,
+                                                volatile int* abort_flag) {
+  const bool r0 = mbar_try_wait(b0, p0), r1 = mbar_try_wait(b1, p1), r2 = mbar_try_wait(b2, p2);
+  if (__builtin_expect(__all_sync(0xffffffffu, r0 && r1 && r2), 1)) return true;
+  return mbar_wait_rest(b0, p0, abort_flag) && mbar_wait_rest(b1, p1, abort_flag) && mbar_wait_rest(b2, p2, abort_flag);
+}
+
 struct TcPlan {
   int n_rest, n_win, nvert0, nvert1, nheads;
   __device__ __forceinline__ int nvert(int h) const { return h ? nvert1 : nvert0; }
@@ -97,6 +119,12 @@ struct TcItemIter {
     if (kind == 0 && j + 1 < pl.n_rest) { ++j; return; }
     if (kind == 2) { if (++j >= pl.n_win) kind = 3; return; }
     do step(pl); while (kind < 3 && !valid(pl));
+  }
+  // at the item behind INT8 tile `last`, whose slot and parity the caller has counted
+  __device__ __forceinline__ void resume(const TcPlan& pl, int last, int slot, uint32_t parity) {
+    kind = 0; j = last; hh = 0;
+    do step(pl); while (kind < 3 && !valid(pl));
+    stage = slot; par = parity;
   }
   __device__ __forceinline__ bool done() const { return kind >= 3; }
   __device__ __forceinline__ bool feeds(int h) const { return kind != 1 || hh == h; }
@@ -355,7 +383,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap mQi, const __grid_constant
       constexpr uint32_t idesc_qk = tc::make_idesc(1, tc::kFmtBF16, tc::kFmtBF16, 128, 64);
       constexpr uint32_t idesc_pv = tc::make_idesc(1, tc::kFmtBF16, tc::kFmtBF16, 128, 128);
       constexpr uint32_t idesc_pv8 = tc::make_idesc(1, tc::kFmtE4M3, tc::kFmtE4M3, 128, 128);
-      auto wait = [&](uint64_t* bar, uint32_t par) { return (bool)__all_sync(0xffffffffu, tc::mbar_wait_abortable(bar, par, abort_flag)); };
+      auto wait = [&](uint64_t* bar, uint32_t par) { return mbar_wait_warp(bar, par, abort_flag); };
       bool ok = wait(q_full, 0);
       // operand descriptors differ only in their start-address field (16-byte units)
       const uint64_t dQi = tc::smem_desc_k128(smem + TcSmem::Qi + h * 16384, 0);
@@ -363,7 +391,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap mQi, const __grid_constant
       const uint64_t dK = tc::smem_desc_k128(smem + TcSmem::K, 0);
       const uint64_t dV = kFp8 ? tc::smem_desc_k64(smem + TcSmem::V, 0) : tc::smem_desc_k128(smem + TcSmem::V, 0);
       const uint32_t tS = tmem_base + kColS + 128u * h, tO = tmem_base + kColO + 128u * h;
-      const int n_t = plan.n_tiles(h);
+      const int n_t = plan.n_tiles(h), n_rest = plan.n_rest;
       TcItemIter cq, cp;
       cq.begin(plan, kKStages);
       cp.begin(plan, kVStages);
@@ -383,6 +411,19 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap mQi, const __grid_constant
           if (tc::elect_one()) tc::mbar_arrive(v_empty + cp.stage);
           cp.next(plan);
         }
+      };
+      auto pv_issue = [&](int t, int stage) {    // one lane
+        const uint32_t aP = tS + 64u * (t & 1);
+        const uint64_t bV = dV + (uint64_t)(stage * 1024);
+        if constexpr (kFp8) {     // 64 keys = two K steps of 32 e4m3: 8 columns of P, 32 bytes of a V^T row each
+#pragma unroll
+          for (int k = 0; k < 2; ++k) tc::mma_f8_ts(tO, aP + 8 * k, bV + 2 * k, idesc_pv8, (t > 0 || k > 0) ? 1u : 0u);
+        } else {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) tc::mma_bf16_ts(tO, aP + 8 * k, bV + 2 * k, idesc_pv, (t > 0 || k > 0) ? 1u : 0u);
+        }
+        tc::mma_commit(pv_done + 2 * h + (t & 1));
+        tc::mma_commit(v_empty + stage);
       };
       auto qk_issue = [&]() {    // one lane
         const uint32_t dS = tS + 64u * (tq & 1);
@@ -424,6 +465,32 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap mQi, const __grid_constant
           cq.next(plan);
         }
         if (!ok) break;
+        // INT8 tiles whose successor but one is INT8 too: tiles and items are the same, nothing to hand back
+        if (t == 0 && tq == 2 && n_rest > 2) {
+          int ks = cq.stage, vs = 0;
+          uint32_t kpar = cq.par, vpar = 0u;
+          for (; t + 2 < n_rest; ++t) {
+            const int sl = 2 * h + (t & 1);
+            ok = mbar_wait_warp3(v_full + vs, vpar, k_full + ks, kpar, p_ready + sl, (uint32_t)((t >> 1) & 1), abort_flag);
+            if (!ok) break;
+            tc::fence_after_sync();
+            if (tc::elect_one()) {
+              pv_issue(t, vs);
+              const uint32_t dS = tS + 64u * (t & 1);
+              const uint64_t bK = dK + (uint64_t)(ks * 1024);
+#pragma unroll
+              for (int k = 0; k < 4; ++k) tc::mma_s8_ss(dS, dQi + 2 * k, bK + 2 * k, idesc_i8, k > 0);
+              tc::mma_commit(s_full + sl);
+              tc::mma_commit(k_empty + ks);
+            }
+            if (++ks == kKStages) { ks = 0; kpar ^= 1u; }
+            if (++vs == kVStages) { vs = 0; vpar ^= 1u; }
+          }
+          if (!ok) break;
+          tq = t + 2;
+          cq.resume(plan, tq - 1, ks, kpar);
+          cp.resume(plan, t - 1, vs, vpar);
+        }
         for (; t < tq; ++t) {
           // the operands first, P last: from the moment P is there nothing is waited for, and P V of t and Q K^T of t + 2
           // are issued together (a wait costs the warp some 400 clocks even if what it waits for is there: 32K hybrid
@@ -438,18 +505,8 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap mQi, const __grid_constant
           ok = wait(p_ready + sl, (uint32_t)((t >> 1) & 1));
           if (!ok) break;
           tc::fence_after_sync();
-          const uint32_t aP = tS + 64u * (t & 1);
-          const uint64_t bV = dV + (uint64_t)(cp.stage * 1024);
           if (tc::elect_one()) {
-            if constexpr (kFp8) {     // 64 keys = two K steps of 32 e4m3: 8 columns of P, 32 bytes of a V^T row each
-#pragma unroll
-              for (int k = 0; k < 2; ++k) tc::mma_f8_ts(tO, aP + 8 * k, bV + 2 * k, idesc_pv8, (t > 0 || k > 0) ? 1u : 0u);
-            } else {
-#pragma unroll
-              for (int k = 0; k < 4; ++k) tc::mma_bf16_ts(tO, aP + 8 * k, bV + 2 * k, idesc_pv, (t > 0 || k > 0) ? 1u : 0u);
-            }
-            tc::mma_commit(pv_done + sl);
-            tc::mma_commit(v_empty + cp.stage);
+            pv_issue(t, cp.stage);
             if (more) qk_issue();
           }
           cp.next(plan);
@@ -483,7 +540,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap mQi, const __grid_constant
       // faster either: 16K 2946 us, with load and wait around the hand-over 3208, like this 2936.)
       uint32_t sr[64];
       auto fetch = [&](int t) {
-        ok = __all_sync(0xffffffffu, tc::mbar_wait_abortable(s_full + 2 * h + (t & 1), (uint32_t)((t >> 1) & 1), abort_flag));
+        ok = mbar_wait_warp(s_full + 2 * h + (t & 1), (uint32_t)((t >> 1) & 1), abort_flag);
         if (!ok) return;
         tc::fence_after_sync();
         tc::tmem_ld32(lane_base + colS + (t & 1) * 64, *reinterpret_cast<uint32_t(*)[32]>(&sr[0]));
@@ -574,12 +631,12 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap mQi, const __grid_constant
       // threads per row, sixteen softmax warps in all: 10.1 ms - the loop lives on shared-memory bandwidth, of which
       // the key scales and biases of 256 rows take 1024 clocks of some 2200 per pair of tiles and the operands of
       // the products 640, and on the issuing warps' latency, which more warps lengthen.)
-      for (int t = 0; t < n_tiles; ++t) {
+      auto tile = [&](int t, auto int8_tile) {
+        constexpr bool is_i8 = decltype(int8_tile)::value;
         const int slot = t & 1, sl = 2 * h + slot;
-        ok = __all_sync(0xffffffffu, tc::mbar_wait_abortable(s_full + sl, (uint32_t)((t >> 1) & 1), abort_flag));
-        if (!ok) break;
+        ok = mbar_wait_warp(s_full + sl, (uint32_t)((t >> 1) & 1), abort_flag);
+        if (!ok) return;
         tc::fence_after_sync();
-        const bool is_i8 = t < n_rest;
         const float esc = is_i8 ? qs : p.sml;                  // > 0
         const float4* ks4 = reinterpret_cast<const float4*>(smem + TcSmem::Ks + ks_slot * kKsBytes);
         const float4* kb4 = ks4 + 16 + 16 * h;
@@ -607,7 +664,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap mQi, const __grid_constant
           const float mu = m_ref == -INFINITY ? 0.f : m_ref;
           const float2 esc2 = make_float2(esc, esc), nmu2 = make_float2(-mu, -mu);
           float2 rsa = make_float2(0.f, 0.f), rsb = make_float2(0.f, 0.f);
-          if (is_i8) {
+          if constexpr (is_i8) {
             float* y = reinterpret_cast<float*>(sr);
 #pragma unroll
             for (int c4 = 0; c4 < 16; ++c4) {
@@ -650,14 +707,14 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap mQi, const __grid_constant
           lsum = (rsa.x + rsa.y) + (rsb.x + rsb.y);
         }
         const bool need = m_ref == -INFINITY || !(lsum <= 256.f);
-        if (__any_sync(0xffffffffu, need)) {
+        if (__builtin_expect(__any_sync(0xffffffffu, need), 0)) {
           // out of line: the maximum, the move of the reference and the tile's P against the new reference
           const bool wait_pv = t > 0;
           const TcSlowResult sr2 = tc_slow_tile(lane_base + colS + slot * 64, lane_base + colO, ks4, kb4, is_i8, esc, mlo, mhi, m_ref, l,
                                                 wait_pv ? pv_done + 2 * h + ((t - 1) & 1) : nullptr, (uint32_t)(((t - 1) >> 1) & 1),
                                                 abort_flag);
           ok = sr2.ok;
-          if (!ok) break;
+          if (!ok) return;
           m_ref = sr2.m_ref;
           l = sr2.l;
         } else {
@@ -668,7 +725,10 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap mQi, const __grid_constant
         }
         tc::fence_before_sync();
         tc::mbar_arrive(p_ready + sl);
-      }
+      };
+      int t = 0;
+      for (; ok && t < n_rest && t < n_tiles; ++t) tile(t, TcTrue{});
+      for (; ok && t < n_tiles; ++t) tile(t, TcFalse{});
     }
     // ---- epilogue: O / l
     if (ok && n_tiles > 0)

@@ -15,11 +15,15 @@ namespace hq {
 constexpr int kReorgWarps = 8;
 constexpr int kReorgTile = 128;   // source rows per CTA
 
-__device__ __forceinline__ int lower_bound_i32(const int32_t* a, int n, int v) {
-  int lo = 0, hi = n;
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    if (__ldg(a + mid) < v) lo = mid + 1; else hi = mid;
+// entries of the ascending list a[0 .. n) below v, by a warp: 32 probes a round (a thread's binary search was eleven loads one after
+// the other at 1600 entries)
+__device__ __forceinline__ int warp_lower_bound(const int32_t* a, int n, int v, int lane) {
+  int lo = 0, len = n;                       // the answer lies in lo .. lo + len
+  while (len > 0) {
+    const int step = (len + 31) / 32, at = lo + (lane + 1) * step - 1;          // the last entry of the lane's part
+    const int below = __popc(__ballot_sync(0xffffffffu, at < lo + len && __ldg(a + at) < v));
+    lo += below * step;
+    len = min(step - 1, n - lo);             // the part that was not below as a whole, without its last entry
   }
   return lo;
 }
@@ -38,8 +42,8 @@ cache_reorg_kernel(const __nv_bfloat16* __restrict__ keys, const __nv_bfloat16* 
                    uint8_t* __restrict__ k_packed, uint8_t* __restrict__ v_packed, int64_t kp_stride_bh, int64_t vp_stride_bh,
                    __half* __restrict__ k_scale, __half* __restrict__ v_scale, int64_t scale_stride_bh,
                    int k_bits, int v_bits, int scale_mode, int prefix_tiles, int topk_tiles) {
-  __shared__ int32_t s_slice[kReorgTile];
-  __shared__ int s_lo, s_hi;
+  __shared__ uint32_t s_bits[kReorgTile / 32];
+  __shared__ int s_range[2];
   const int bh = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const __nv_bfloat16* K = keys + bh * kv_stride_bh;
   const __nv_bfloat16* V = values + bh * kv_stride_bh;
@@ -47,40 +51,54 @@ cache_reorg_kernel(const __nv_bfloat16* __restrict__ keys, const __nv_bfloat16* 
   if (tile < prefix_tiles) {
     const int p0 = tile * kReorgTile, p1 = min(p0 + kReorgTile, prefix_len);
     const int32_t* asc = vidx_asc + (int64_t)bh * T;
-    if (threadIdx.x == 0) {
-      s_lo = T > 0 ? lower_bound_i32(asc, T, p0) : 0;
-      s_hi = T > 0 ? lower_bound_i32(asc, T, p1) : 0;
+    // eight lanes per source row, four rows per warp and trip (every lane stays in step for the shuffles); a trip's rows are
+    // asked for while the one before is quantised, the first before the block looks up its part of the list
+    const int sub = lane & 7;
+    struct Raw { uint4 k[2], v[2]; };
+    auto fetch = [&](int pb, Raw& r) {
+      const int64_t at = (int64_t)min(pb + (lane >> 3), p1 - 1) * 128 + sub * 16;
+      r.k[0] = __ldg(reinterpret_cast<const uint4*>(K + at)); r.k[1] = __ldg(reinterpret_cast<const uint4*>(K + at) + 1);
+      r.v[0] = __ldg(reinterpret_cast<const uint4*>(V + at)); r.v[1] = __ldg(reinterpret_cast<const uint4*>(V + at) + 1);
+    };
+    Raw next;
+    fetch(p0 + 4 * warp, next);
+    // the tile's vertical rows as bits, and how many lie below each of its words
+    if (warp < 2) {
+      const int at = T > 0 ? warp_lower_bound(asc, T, warp ? p1 : p0, lane) : 0;
+      if (lane == 0) s_range[warp] = at;
+    }
+    if (threadIdx.x < kReorgTile / 32) s_bits[threadIdx.x] = 0u;
+    __syncthreads();
+    const int lo = s_range[0], cnt = s_range[1] - lo;   // cnt <= rows in tile (indices are distinct)
+    for (int i = threadIdx.x; i < cnt; i += blockDim.x) {
+      const unsigned o = (unsigned)(__ldg(asc + lo + i) - p0);
+      if (o < kReorgTile) atomicOr(&s_bits[o >> 5], 1u << (o & 31));
     }
     __syncthreads();
-    const int lo = s_lo, cnt = s_hi - s_lo;   // cnt <= rows in tile (indices are distinct)
-    for (int i = threadIdx.x; i < cnt; i += blockDim.x) s_slice[i] = __ldg(asc + lo + i);
-    __syncthreads();
     const int n_quant = prefix_len - T;
-    // eight lanes per source row, four rows per warp and trip (every lane stays in step for the shuffles)
-    const int sub = lane & 7;
-    for (int pb = p0 + 4 * warp; pb < p1; pb += 4 * kReorgWarps) {
-      const int p = pb + (lane >> 3);
-      // rank within the slice: entries < p; hit: an entry == p
-      int below = 0, hit = 0;
-      for (int i = sub; i < cnt; i += 8) {
-        const int v = s_slice[i];
-        below += v < p;
-        hit |= v == p;
-      }
+    int distinct = 0;
 #pragma unroll
-      for (int o = 4; o > 0; o >>= 1) {
-        below += __shfl_xor_sync(0xffffffffu, below, o);
-        hit |= __shfl_xor_sync(0xffffffffu, hit, o);
+    for (int w = 0; w < kReorgTile / 32; ++w) distinct += __popc(s_bits[w]);
+    for (int pb = p0 + 4 * warp; pb < p1; pb += 4 * kReorgWarps) {
+      const Raw cur = next;
+      if (pb + 4 * kReorgWarps < p1) fetch(pb + 4 * kReorgWarps, next);
+      const int p = pb + (lane >> 3), o = p - p0;
+      int below = 0;
+#pragma unroll
+      for (int w = 0; w < kReorgTile / 32; ++w) below += __popc(s_bits[w] & (o >= 32 * w + 32 ? 0xFFFFFFFFu : o >= 32 * w ? (1u << (o & 31)) - 1u : 0u));
+      if (distinct != cnt) {                 // a list with repeated rows: every entry counts
+        below = 0;
+        for (int i = 0; i < cnt; ++i) below += __ldg(asc + lo + i) < p;
       }
+      const bool hit = p < p1 && ((s_bits[(o >> 5) & (kReorgTile / 32 - 1)] >> (o & 31)) & 1u);
       const int dst = p - (lo + below);
       const bool live = p < p1 && !hit && dst >= 0 && dst < n_quant;     // dst out of range cannot happen for a consistent index list
-      const int ps = p < p1 ? p : p1 - 1;
-      float kv[16], vv[16];
-      load16(K + (int64_t)ps * 128 + sub * 16, kv);
-      load16(V + (int64_t)ps * 128 + sub * 16, vv);
       const int64_t d = live ? dst : 0;
-      const __half sk = quant_store_row16(k_bits, kv, scale_mode, k_packed + bh * kp_stride_bh + d * (16 * k_bits), sub, live);
-      const __half sv = quant_store_row16(v_bits, vv, scale_mode, v_packed + bh * vp_stride_bh + d * (16 * v_bits), sub, live);
+      float x[16];
+      unpack16(cur.k[0], cur.k[1], x);
+      const __half sk = quant_store_row16(k_bits, x, scale_mode, k_packed + bh * kp_stride_bh + d * (16 * k_bits), sub, live);
+      unpack16(cur.v[0], cur.v[1], x);
+      const __half sv = quant_store_row16(v_bits, x, scale_mode, v_packed + bh * vp_stride_bh + d * (16 * v_bits), sub, live);
       if (live && sub == 0) {
         k_scale[bh * scale_stride_bh + dst] = sk;
         v_scale[bh * scale_stride_bh + dst] = sv;

@@ -13,6 +13,7 @@
 // thread in flight, and kept in shared memory; three-pass radix select of the k-th largest key with a scan over the
 // bins, order-preserving compaction (ties go to the lower index; it is also the ascending list), bitonic sort of the
 // selected (key, ~index) pairs, the short distances inside warps.
+#include <cooperative_groups.h>
 #include "hq_common.cuh"
 
 namespace hq {
@@ -375,6 +376,277 @@ topk_kernel(const float* __restrict__ scores, int64_t stride, int n, int k, int 
     idx_desc[(int64_t)blockIdx.x * k + i] = (int64_t)(~(uint32_t)(sel[i] & 0xFFFFFFFFull));
 }
 
+// ---- the same for long rows
+constexpr int kSliceThreads = 512, kSliceWarps = kSliceThreads / 32;
+constexpr int kTopkCluster = 8;            // most blocks per row
+
+__device__ __forceinline__ int warp_inclusive_scan(int v) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int n = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= o) v += n;
+  }
+  return v;
+}
+
+__device__ __forceinline__ int slice_exclusive_scan(int v, int* warp_sums) {
+  // kSliceThreads threads; returns the exclusive prefix of v over the block
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int inc = warp_inclusive_scan(v);
+  __syncthreads();               // protect warp_sums reuse
+  if (lane == 31) warp_sums[warp] = inc;
+  __syncthreads();
+  int before = lane < warp ? warp_sums[lane] : 0;               // kSliceWarps <= 32
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+  return before + inc - v;
+}
+
+// A row is taken by a cluster of blocks, each with a contiguous slice of it.  Radix select: every block counts its slice's
+// digits, adds up the cluster's counters over distributed shared memory and finds the same digit; then it keeps what it has
+// above the threshold (and its share of what equals it) in index order, sorts that, and an entry's place in the whole list
+// is its own plus, for every other block, the entries above it there (a binary search).  8 rows of 32K candidates: 36 us
+// with a block each (counting 20 K clocks, compaction 14 K, the sort 18 K of 74 K), 19 us this way.
+// kCached: the slice's keys stay in shared memory after the first pass (up to some 50 thousand); longer slices are read again.
+template <bool kCached>
+__global__ void __launch_bounds__(kSliceThreads)
+topk_cluster_kernel(const float* __restrict__ scores, int64_t stride, int n, int k, int seg, int selcap,
+            int64_t* __restrict__ idx_desc, int32_t* __restrict__ idx_asc) {
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  unsigned long long* sel = reinterpret_cast<unsigned long long*>(smem_raw);   // [selcap]
+  int* hist = reinterpret_cast<int*>(sel + selcap);                            // [2][kTopkBins]
+  uint32_t* keys = reinterpret_cast<uint32_t*>(hist + 2 * kTopkBins);          // [seg] if kCached
+  __shared__ int warp_sums[kSliceWarps];
+  __shared__ __align__(8) int s_sums[2][kTopkBins / 32];
+  __shared__ uint32_t s_bin;
+  __shared__ int s_remaining;
+  __shared__ int s_count[2];                                                   // above T, equal to T
+  __shared__ int s_off[kTopkCluster + 1];                                      // where the blocks' entries begin in the ascending list
+  namespace cg = cooperative_groups;
+  const cg::cluster_group cluster = cg::this_cluster();
+  const int blocks = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t r = blockIdx.x / blocks;
+  const int first = min(rank * seg, n), m = min(first + seg, n) - first;       // the slice: first .. first + m
+  const float* row = scores + r * stride + first;
+  auto key_at = [&](int i) -> uint32_t { return kCached ? keys[i] : orderable(__ldg(row + i)); };
+
+  // ---- radix select: find key T of the k-th largest element (digits of 11, 11 and 10 bits)
+  uint32_t prefix = 0, mask = 0;
+  int remaining = k;   // rank (1-based from the top) within the current candidate set
+#pragma unroll 1
+  for (int pass = 0; pass < 3; ++pass) {
+    const int shift = pass == 0 ? 21 : pass == 1 ? 10 : 0;
+    const uint32_t digits = pass == 2 ? 1023u : 2047u;
+    // the counters of two passes ago: the cluster has met since their last reader
+    int* h = hist + (pass & 1) * kTopkBins;
+    *reinterpret_cast<int4*>(h + 4 * tid) = make_int4(0, 0, 0, 0);
+    __syncthreads();
+    for (int i0 = tid; i0 < m; i0 += 8 * kSliceThreads) {
+      uint32_t key[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int i = i0 + j * kSliceThreads;
+        key[j] = i < m ? ((kCached && pass > 0) ? keys[i] : orderable(__ldg(row + i))) : 0u;
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int i = i0 + j * kSliceThreads;
+        if (i < m) {
+          if (kCached && pass == 0) keys[i] = key[j];
+          if ((key[j] & mask) == prefix) atomicAdd(&h[(key[j] >> shift) & digits], 1);
+        }
+      }
+    }
+    __syncthreads();
+    // sums of 32 counters, so that the cluster's are first added up 64 sums and then 32 counters at a time (all 2048 of
+    // every block: 4400 clocks a pass at 8 blocks, now 1700)
+    int* sums = s_sums[pass & 1];
+    for (int x = warp; x < kTopkBins / 32; x += kSliceWarps) {
+      const int v = __reduce_add_sync(0xffffffffu, h[32 * x + lane]);
+      if (lane == 0) sums[x] = v;
+    }
+    cluster.sync();
+    // the digit that holds the wanted rank: the group of bins (lane l has groups 63 - 2 l and 62 - 2 l), then the bin
+    if (warp == 0) {
+      int2 c = make_int2(0, 0);
+#pragma unroll
+      for (int b = 0; b < kTopkCluster; ++b) {                   // all loads in flight together
+        if (b < blocks) {
+          const int2 x = *reinterpret_cast<const int2*>(cluster.map_shared_rank(sums, b) + 62 - 2 * lane);
+          c.x += x.x; c.y += x.y;
+        }
+      }
+      int upto = warp_inclusive_scan(c.x + c.y);
+      int above = upto - c.x - c.y;
+      const int at = __ffs(__ballot_sync(0xffffffffu, above < remaining && remaining <= upto)) - 1;
+      const bool high = remaining <= above + c.y;
+      const int group = __shfl_sync(0xffffffffu, high ? 63 - 2 * lane : 62 - 2 * lane, at);
+      const int left = remaining - __shfl_sync(0xffffffffu, high ? above : above + c.y, at);
+      int n_bin = 0;
+#pragma unroll
+      for (int b = 0; b < kTopkCluster; ++b)
+        if (b < blocks) n_bin += cluster.map_shared_rank(h, b)[32 * group + 31 - lane];
+      upto = warp_inclusive_scan(n_bin);
+      if (upto - n_bin < left && left <= upto) {
+        s_bin = (uint32_t)(32 * group + 31 - lane);
+        s_remaining = left - (upto - n_bin);
+      }
+    }
+    __syncthreads();
+    prefix |= s_bin << shift;
+    remaining = s_remaining;
+    mask |= digits << shift;
+  }
+  const uint32_t T = prefix;        // threshold key
+  const int need_eq = remaining;    // how many elements equal to T to take (lowest indices first)
+
+  // ---- order-preserving compaction into sel[]: warp w owns one contiguous range of the slice, counts what it has and
+  // writes once the warps and blocks before it are known; the order of the list is the ascending index list
+  const int wseg = ((seg + kSliceWarps - 1) / kSliceWarps + 31) & ~31;
+  const int s0 = min(warp * wseg, m), s1 = min(s0 + wseg, m);
+  int gt = 0, eq = 0;
+  for (int i = s0 + lane; i < s1; i += 32) {
+    const uint32_t key = key_at(i);
+    gt += key > T;
+    eq += key == T;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    gt += __shfl_xor_sync(0xffffffffu, gt, o);
+    eq += __shfl_xor_sync(0xffffffffu, eq, o);
+  }
+  const int eq_scan = slice_exclusive_scan(lane == 0 ? eq : 0, warp_sums);
+  const int gt_scan = slice_exclusive_scan(lane == 0 ? gt : 0, warp_sums);
+  if (tid == kSliceThreads - 32) { s_count[0] = gt_scan + gt; s_count[1] = eq_scan + eq; }
+  cluster.sync();
+  // lane b: block b's counts, and what the blocks before it have of either and keep
+  int b_gt = 0, b_eq = 0;
+  if (lane < blocks) {
+    const int* c = cluster.map_shared_rank(s_count, lane);
+    b_gt = c[0];
+    b_eq = c[1];
+  }
+  int gt_upto = b_gt, eq_upto = b_eq;
+#pragma unroll
+  for (int o = 1; o < kTopkCluster; o <<= 1) {
+    const int x = __shfl_up_sync(0xffffffffu, gt_upto, o), y = __shfl_up_sync(0xffffffffu, eq_upto, o);
+    if (lane >= o) { gt_upto += x; eq_upto += y; }
+  }
+  const int b_end = gt_upto + min(eq_upto, need_eq);
+  if (warp == 0 && lane < blocks) s_off[lane + 1] = b_end;
+  if (tid == 0) s_off[0] = 0;
+  const int gt_before = __shfl_sync(0xffffffffu, gt_upto - b_gt, rank), eq_before = __shfl_sync(0xffffffffu, eq_upto - b_eq, rank);
+  const int out0 = gt_before + min(eq_before, need_eq);         // the block's place in the ascending list
+  int eq_seen = eq_before + __shfl_sync(0xffffffffu, eq_scan, 0);            // == T elements of the blocks and warps before
+  int out_pos = gt_before + __shfl_sync(0xffffffffu, gt_scan, 0) + min(eq_seen, need_eq) - out0;
+  const int kept = __shfl_sync(0xffffffffu, b_end, rank) - out0;
+  if (gt + max(0, min(eq, need_eq - eq_seen)) > 0) {
+    const uint32_t lt = (1u << lane) - 1u;
+    for (int i0 = s0; i0 < s1; i0 += 32) {
+      const int i = i0 + lane;
+      const uint32_t key = i < s1 ? key_at(i) : 0u;
+      const bool is_eq = i < s1 && key == T;
+      const uint32_t eqs = __ballot_sync(0xffffffffu, is_eq);
+      const bool take = i < s1 && (key > T || (is_eq && eq_seen + __popc(eqs & lt) < need_eq));
+      const uint32_t takes = __ballot_sync(0xffffffffu, take);
+      if (take) {
+        const int pos = out_pos + __popc(takes & lt);
+        sel[pos] = ((unsigned long long)key << 32) | (uint32_t)(~(uint32_t)(first + i));
+        if (idx_asc) idx_asc[r * k + out0 + pos] = first + i;
+      }
+      eq_seen += __popc(eqs);
+      out_pos += __popc(takes);
+    }
+  }
+  int kpad = 64;
+  while (kpad < kept) kpad <<= 1;                               // <= selcap
+  for (int i = kept + tid; i < kpad; i += kSliceThreads) sel[i] = 0ull;   // smaller than any real entry
+  __syncthreads();
+
+  // ---- bitonic sort, descending: distances of 64 and more through shared memory, the rest inside warps
+  for (int base = warp * 64; base < kpad; base += kSliceWarps * 64) {
+    unsigned long long a = sel[base + lane], c = sel[base + 32 + lane];
+    for (int size = 2; size <= 64; size <<= 1) bitonic_in_warp(a, c, base, lane, size, size >> 1);
+    sel[base + lane] = a; sel[base + 32 + lane] = c;
+  }
+  __syncthreads();
+  for (int size = 128; size <= kpad; size <<= 1) {
+    for (int strd = size >> 1; strd >= 64; strd >>= 1) {
+      for (int x = tid; x < (kpad >> 1); x += kSliceThreads) {
+        const int lo = 2 * x - (x & (strd - 1));
+        const int hi = lo + strd;
+        const bool desc = ((lo & size) == 0);
+        const unsigned long long a = sel[lo], b2 = sel[hi];
+        if ((a < b2) == desc) { sel[lo] = b2; sel[hi] = a; }
+      }
+      __syncthreads();
+    }
+    for (int base = warp * 64; base < kpad; base += kSliceWarps * 64) {
+      unsigned long long a = sel[base + lane], c = sel[base + 32 + lane];
+      bitonic_in_warp(a, c, base, lane, size, 32);
+      sel[base + lane] = a; sel[base + 32 + lane] = c;
+    }
+    __syncthreads();
+  }
+
+  // ---- places: entries are distinct (the index is part of them), so the lists of the blocks interleave without ties.  All
+  // lists are brought over where the counters and keys, which are done with, leave room for them (k of up to an eighth of
+  // the row's slices and 2048 besides), and the searches of an entry run side by side.
+  cluster.sync();
+  if (blocks > 1 && (size_t)k * 8 <= 2 * kTopkBins * sizeof(int) + (kCached ? (size_t)seg * 4 : 0)) {
+    unsigned long long* all = reinterpret_cast<unsigned long long*>(hist);
+    int longest = 0;
+#pragma unroll
+    for (int b = 0; b < kTopkCluster; ++b)
+      if (b < blocks) longest = max(longest, s_off[b + 1] - s_off[b]);
+#pragma unroll 4
+    for (int x = tid; x < k; x += kSliceThreads) {
+      int b = 0;
+#pragma unroll
+      for (int c = 1; c < kTopkCluster; ++c) b += c < blocks && x >= s_off[c];
+      all[x] = cluster.map_shared_rank(sel, b)[x - s_off[b]];
+    }
+    __syncthreads();
+    int top = 1;
+    while (2 * top <= longest) top <<= 1;
+    for (int i = tid; i < kept; i += kSliceThreads) {
+      const unsigned long long e = sel[i];
+      int pos[kTopkCluster] = {};                                // entries above e in the block's list
+      for (int step = top; step > 0; step >>= 1) {
+#pragma unroll
+        for (int b = 0; b < kTopkCluster; ++b)
+          if (b < blocks) {
+            const int at = s_off[b] + pos[b] + step;
+            if (at <= s_off[b + 1] && all[at - 1] > e) pos[b] += step;
+          }
+      }
+      int place = 0;
+#pragma unroll
+      for (int b = 0; b < kTopkCluster; ++b) place += pos[b];
+      idx_desc[r * k + place] = (int64_t)(~(uint32_t)(e & 0xFFFFFFFFull));
+    }
+  } else {
+    for (int i = tid; i < kept; i += kSliceThreads) {
+      const unsigned long long e = sel[i];
+      int place = i;
+      for (int d = 1; d < blocks; ++d) {
+        const int b = (rank + d) % blocks;
+        const unsigned long long* other = cluster.map_shared_rank(sel, b);
+        int lo = 0, hi = s_off[b + 1] - s_off[b];
+        while (lo < hi) {
+          const int mid = (lo + hi) >> 1;
+          if (other[mid] > e) lo = mid + 1; else hi = mid;
+        }
+        place += lo;
+      }
+      idx_desc[r * k + place] = (int64_t)(~(uint32_t)(e & 0xFFFFFFFFull));
+    }
+  }
+  cluster.sync();                   // a block's lists stay until the others have read them
+}
+
 }  // namespace hq
 
 namespace hq {
@@ -465,7 +737,33 @@ extern "C" int hq_topk(const float* scores, int64_t scores_stride, int rows, int
   if (attr_dev != dev) {
     HQ_CUDA(cudaFuncSetAttribute(topk_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem));
     HQ_CUDA(cudaFuncSetAttribute(topk_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem));
+    HQ_CUDA(cudaFuncSetAttribute(topk_cluster_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem));
+    HQ_CUDA(cudaFuncSetAttribute(topk_cluster_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem));
     attr_dev = dev;
+  }
+  // A cluster per row from 12K candidates on, with slices of 2K or more and no more blocks than two to an SM.  Measured (us, block /
+  // cluster): 8 or 32 rows of 8K 13.3 / 14.2, 64 of 16K 21.1 / 19.7 (four blocks; eight 25.3), 8 of 32K 36.3 / 19.2, 32 of 32K
+  // 36.4 / 23.4, 2 of 128K 146 / 41.
+  int blocks = kTopkCluster;
+  while (blocks > 1 && (n < 2048 * blocks || (int64_t)rows * blocks > 2 * sm_count())) blocks >>= 1;
+  if (n >= 12288 && blocks > 1) {
+    const int seg = ((n + blocks - 1) / blocks + 31) & ~31;
+    int selcap = 64;
+    while (selcap < (k < seg ? k : seg)) selcap <<= 1;
+    const size_t slice_need = (size_t)selcap * 8 + 2 * kTopkBins * 4, slice_keys = slice_need + (size_t)seg * 4;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)rows * blocks);
+    cfg.blockDim = dim3(kSliceThreads);
+    cfg.dynamicSmemBytes = slice_keys <= kMaxSmem ? slice_keys : slice_need;
+    cfg.stream = (cudaStream_t)stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)blocks; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    if (slice_keys <= kMaxSmem) HQ_CUDA(cudaLaunchKernelEx(&cfg, topk_cluster_kernel<true>, scores, scores_stride, n, k, seg, selcap, idx_desc, idx_asc));
+    else HQ_CUDA(cudaLaunchKernelEx(&cfg, topk_cluster_kernel<false>, scores, scores_stride, n, k, seg, selcap, idx_desc, idx_asc));
+    return HQ_OK;
   }
   if (with_keys <= kMaxSmem)
     topk_kernel<true><<<rows, kTopkThreads, with_keys, (cudaStream_t)stream>>>(scores, scores_stride, n, k, kpad, idx_desc, idx_asc);

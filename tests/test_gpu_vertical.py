@@ -178,3 +178,76 @@ def test_cache_reorganize_bit_exact(BH, N, W, T):
     assert np.array_equal(layer.k_window.float().cpu().numpy(), oc.k_window)
     assert np.array_equal(layer.v_window.float().cpu().numpy(), oc.v_window)
     assert layer._staging_buf_k.shape == (BH, 128, 128) and float(layer._staging_buf_k.abs().sum()) == 0.0
+
+
+@pytest.mark.parametrize("rows,n,k,kind", [(3, 12288, 614, "normal"), (2, 12289, 1, "normal"), (1, 16384, 16384, "ties"), (5, 20011, 1000, "ties"),
+                                           (2, 32512, 1625, "one slice"), (70, 12301, 77, "normal"), (1, 131071, 6553, "normal"),
+                                           (2, 40000, 9000, "infinities"), (1, 400001, 300, "normal")])
+def test_topk_of_long_rows(rows, n, k, kind):
+    """Rows that a cluster of blocks shares: odd slices, ties across slices, everything in one slice, lists too long to be
+    brought together, slices too long to be kept; the same list as the oracle's, bit for bit."""
+    rng = np.random.default_rng(n + k)
+    s = rng.standard_normal((rows, n)).astype(np.float32)
+    if kind == "ties":
+        s = np.round(2 * s).astype(np.float32)
+    elif kind == "one slice":
+        s[:, 9000:9000 + k] += 100.0
+    elif kind == "infinities":
+        s[:, ::7] = -np.inf
+        s[:, 5::1000] = np.inf
+    idx, asc = hq.topk_indices(torch.from_numpy(s).to(DEV)[None], k, want_ascending=True)
+    want = orc.topk_desc(s[None], k)
+    assert np.array_equal(idx.cpu().numpy(), want)
+    assert np.array_equal(asc.cpu().numpy(), np.sort(want, axis=-1))
+
+
+@pytest.mark.parametrize("N,W,T,dense", [(700, 64, 32, False), (700, 64, 33, False), (5000, 128, 1025, False), (1000, 100, 200, True),
+                                         (129, 1, 127, True), (260, 4, 0, False)])
+def test_reorganisation_places_every_row(N, W, T, dense):
+    """The list search (32 probes a round) and the rank bits at the edges of tiles: vertical rows anywhere, or filling
+    whole tiles; the rest in order, as the quantiser packs it."""
+    g = torch.Generator(device="cpu").manual_seed(N + T)
+    kv = torch.randn(2, 1, 2, N, 128, generator=g).to(torch.bfloat16).to(DEV)
+    P = N - W
+    picks = [torch.arange(3, 3 + T) % P if dense else torch.randperm(P, generator=g)[:T] for _ in range(2)]
+    idx = torch.stack(picks)[None].to(DEV)
+    layer = hq.DStageLayerCache(0, k_bits=4, v_bits=8, window_size=W, use_vert=False)
+    layer.update_prefill(kv[0], kv[1])
+    layer.freeze(1, vertical_indices=idx)
+    for h in range(2):
+        rest = torch.ones(P, dtype=torch.bool)
+        rest[picks[h]] = False
+        for x, bits, packed, scale, topk in ((kv[0], 4, layer.k_quant_packed, layer.k_scale, layer.k_topk), (kv[1], 8, layer.v_quant_packed, layer.v_scale, layer.v_topk)):
+            row = x[0, h]
+            codes, sc = hq.quantize_per_token(row[:P][rest.to(DEV)][None], bits)
+            assert torch.equal(topk[h], row[picks[h].to(DEV)])
+            assert packed.shape[1] == P - T
+            assert torch.equal(packed[h].view(torch.int8), codes[0]) and torch.equal(scale[h].reshape(-1), sc[0])
+
+
+@pytest.mark.parametrize("bits", [2, 4, 8])
+def test_quantiser_words_that_leave_the_common_path(bits):
+    """Rows of subnormal scale (where a quotient can round past q_max), rows full of half-integers, and a NaN or an infinity in
+    one word of a row: the codes of the oracle; a NaN is the lowest code and does not count for the scale."""
+    rng = np.random.default_rng(bits)
+    qmax = 2 ** (bits - 1) - 1
+    x = rng.standard_normal((1, 200, 128)).astype(np.float32)
+    x[0, :60] *= np.geomspace(1e-9, 1e-2, 60)[:, None].astype(np.float32)
+    x[0, 60:140] = (rng.integers(-2 * qmax, 2 * qmax + 1, (80, 128)) * 0.5).astype(np.float32)
+    x[0, 60:140, 5] = qmax                                    # scale 1: every odd half is a tie
+    x = orc.bf16_round(x)
+    for mode in (0, 1):
+        pk = torch.empty(1, 200, 16 * bits, dtype=torch.int8, device=DEV)
+        sc = torch.empty(1, 200, dtype=torch.float16, device=DEV)
+        hq.quantize_per_token_into(t_bf16(x), pk, sc, 0, nbits=bits, scale_mode=mode)
+        po, so = orc.quantize_per_token(x, bits, reciprocal_scale=mode == 1)
+        assert np.array_equal(pk.cpu().numpy(), po) and np.array_equal(sc.cpu().numpy().view(np.uint16), so.view(np.uint16))
+    odd = x[:, 150:152].copy()
+    clean, _ = hq.quantize_per_token(t_bf16(np.where(np.arange(128) == 40, 0, odd)), bits)
+    odd[0, :, 40] = np.nan
+    got, _ = hq.quantize_per_token(t_bf16(odd), bits)
+    per = 8 // bits
+    low = np.uint8(((1 << (bits - 1)) & ((1 << bits) - 1)) << (bits * (40 % per)))
+    want = clean.cpu().numpy().view(np.uint8).copy()
+    want[0, :, 40 // per] |= low
+    assert np.array_equal(got.cpu().numpy().view(np.uint8), want)

@@ -15,6 +15,7 @@
 //
 // Tensor-bound.  FLOPs per call: 4 * B * H_Q * 128 * N (N + 1) / 2.  The attention kernel itself
 // (tcgen05 / tensor memory / TMA) lives in hq_prefill_tc.cu.
+#include <cstddef>
 #include "hq_common.cuh"
 
 namespace hq {
@@ -148,9 +149,9 @@ vertical_sort_kernel(const int64_t* __restrict__ idx, int T, int last, int32_t* 
 }  // namespace hq
 
 namespace hq {
-int prefill_tc_launch(const hq_prefill_args* a, cudaStream_t st);
+int prefill_tc_launch(const hq_prefill_args* a, bool v_rows, cudaStream_t st);
 int prefill_tc_prepare_v(const void* v, int64_t sb, int64_t sh, int64_t sn, int B, int H_KV, int N, void* v_t, cudaStream_t st);
-int prefill_tc_prepare_vertical(const int32_t* vasc, int B, int H_Q, int H_KV, int N, int T, const void* k_bf, const void* v,
+int prefill_tc_prepare_vertical(bool rows, const int32_t* vasc, int B, int H_Q, int H_KV, int N, int T, const void* k_bf, const void* v,
                                 int64_t v_sb, int64_t v_sh, int64_t v_sn, void* xk, void* xvt, cudaStream_t st);
 int prefill_tc_prepare_v_fp8(const void* v, int64_t sb, int64_t sh, int64_t sn, int B, int H_KV, int N, void* v_t8, float* v_scale,
                              void* amax_scratch, cudaStream_t st);
@@ -207,10 +208,10 @@ extern "C" int hq_prefill_vertical_sort(const int64_t* vidx, int rows, int T, in
   return HQ_OK;
 }
 
-extern "C" int hq_prefill_vertical_prepare(const int32_t* vidx_asc, int B, int H_Q, int H_KV, int N, int window, int T,
-                                           const void* k_bf, const void* v, int64_t v_sb, int64_t v_sh, int64_t v_sn,
-                                           const float* k_scale, void* vert_k, void* vert_vt, float* k_bias,
-                                           int32_t* nv_valid, void* stream) {
+static int vertical_prepare(bool rows, const int32_t* vidx_asc, int B, int H_Q, int H_KV, int N, int window, int T,
+                            const void* k_bf, const void* v, int64_t v_sb, int64_t v_sh, int64_t v_sn,
+                            const float* k_scale, void* vert_k, void* vert_vt, float* k_bias,
+                            int32_t* nv_valid, void* stream) {
   using namespace hq;
   HQ_REQUIRE(B > 0 && H_Q > 0 && H_KV > 0 && N > 0 && T >= 0 && window >= 0 && H_Q % H_KV == 0, HQ_ERR_INVALID,
              "hq_prefill_vertical_prepare: bad sizes");
@@ -225,14 +226,33 @@ extern "C" int hq_prefill_vertical_prepare(const int32_t* vidx_asc, int B, int H
   if (T == 0) return HQ_OK;
   HQ_REQUIRE(aligned16(v) && aligned16(k_bf) && aligned16(vert_k) && aligned16(vert_vt) && v_sb % 8 == 0 &&
                  v_sh % 8 == 0 && v_sn % 8 == 0, HQ_ERR_ALIGNMENT, "hq_prefill_vertical_prepare: rows must be 16-byte aligned");
-  return prefill_tc_prepare_vertical(vidx_asc, B, H_Q, H_KV, N, T, k_bf, v, v_sb, v_sh, v_sn, vert_k, vert_vt, st);
+  return prefill_tc_prepare_vertical(rows, vidx_asc, B, H_Q, H_KV, N, T, k_bf, v, v_sb, v_sh, v_sn, vert_k, vert_vt, st);
+}
+
+extern "C" int hq_prefill_vertical_prepare(const int32_t* vidx_asc, int B, int H_Q, int H_KV, int N, int window, int T,
+                                           const void* k_bf, const void* v, int64_t v_sb, int64_t v_sh, int64_t v_sn,
+                                           const float* k_scale, void* vert_k, void* vert_vt, float* k_bias,
+                                           int32_t* nv_valid, void* stream) {
+  return vertical_prepare(false, vidx_asc, B, H_Q, H_KV, N, window, T, k_bf, v, v_sb, v_sh, v_sn, k_scale, vert_k, vert_vt, k_bias,
+                          nv_valid, stream);
+}
+
+extern "C" int hq_prefill_vertical_prepare_rows(const int32_t* vidx_asc, int B, int H_Q, int H_KV, int N, int window, int T,
+                                           const void* k_bf, const void* v, int64_t v_sb, int64_t v_sh, int64_t v_sn,
+                                           const float* k_scale, void* vert_k, void* vert_v, float* k_bias,
+                                           int32_t* nv_valid, void* stream) {
+  return vertical_prepare(true, vidx_asc, B, H_Q, H_KV, N, window, T, k_bf, v, v_sb, v_sh, v_sn, k_scale, vert_k, vert_v, k_bias,
+                          nv_valid, stream);
 }
 
 extern "C" int hq_prefill_hybrid(const hq_prefill_args* a, void* stream) {
   using namespace hq;
   HQ_REQUIRE(a != nullptr, HQ_ERR_INVALID, "hq_prefill_hybrid: null args");
-  HQ_REQUIRE(a->struct_bytes == (int32_t)sizeof(hq_prefill_args), HQ_ERR_INVALID, "hq_prefill_hybrid: struct_bytes %d != %d",
+  // the struct as it was before V's strides is taken too (its flag word was reserved and is not read)
+  const bool short_args = a->struct_bytes == (int32_t)offsetof(hq_prefill_args, v_sb);
+  HQ_REQUIRE(short_args || a->struct_bytes == (int32_t)sizeof(hq_prefill_args), HQ_ERR_INVALID, "hq_prefill_hybrid: struct_bytes %d != %d",
              a->struct_bytes, (int)sizeof(hq_prefill_args));
+  const bool v_rows = !short_args && a->v_rows != 0 && !a->pv_fp8;
   HQ_REQUIRE(a->head_dim == 128, HQ_ERR_UNSUPPORTED, "hq_prefill_hybrid: head_dim %d (only 128 is built)", a->head_dim);
   HQ_REQUIRE(a->B > 0 && a->H_Q > 0 && a->H_KV > 0 && a->N > 0 && a->H_Q % a->H_KV == 0 && a->window >= 0 && a->T >= 0,
              HQ_ERR_INVALID, "hq_prefill_hybrid: bad sizes");
@@ -251,5 +271,10 @@ extern "C" int hq_prefill_hybrid(const hq_prefill_args* a, void* stream) {
              HQ_ERR_ALIGNMENT, "hq_prefill_hybrid: operand rows must be 16-byte aligned");
   HQ_REQUIRE(a->out_dtype == HQ_BF16 || a->out_dtype == HQ_F16 || a->out_dtype == HQ_F32, HQ_ERR_UNSUPPORTED,
              "hq_prefill_hybrid: out_dtype %d", a->out_dtype);
-  return prefill_tc_launch(a, (cudaStream_t)stream);
+  if (v_rows) {
+    HQ_REQUIRE(a->v_sb > 0 && a->v_sh > 0 && a->v_sn > 0 && a->v_sb % 8 == 0 && a->v_sh % 8 == 0 && a->v_sn % 8 == 0, HQ_ERR_ALIGNMENT,
+               "hq_prefill_hybrid: rows of v must be 16-byte aligned");
+    HQ_REQUIRE(a->T == 0 || aligned16(a->vert_vt), HQ_ERR_ALIGNMENT, "hq_prefill_hybrid: vert_vt must be 16-byte aligned");
+  }
+  return prefill_tc_launch(a, v_rows, (cudaStream_t)stream);
 }

@@ -9,12 +9,12 @@
 // interleave on the SM: while one head's threads are in their exponentials the tensor core runs the other
 // head's products.  11 warps:
 //   warp 8 (one lane)  producer: TMA tensor-map loads (128-byte swizzle) of both heads' Q once, then K tiles
-//                      and transposed V tiles into two rings of three and four slots (a K slot is free again
+//                      and V tiles into two rings of three and four slots (a K slot is free again
 //                      after the heads' Q K^T, a V slot after their P V).  INT8 and window items serve both heads;
 //                      the gathered vertical-line tiles are per head.
 //   warps 9, 10        (an elected lane each) issue tcgen05.mma for head A / B: S = Q K^T (kind::i8 with s32
 //                      accumulators, or kind::f16 on bf16) into one of the head's two S buffers in tensor
-//                      memory, two tiles ahead of O += P V (kind::f16, P read from tensor memory, V^T from
+//                      memory, two tiles ahead of O += P V (kind::f16, P read from tensor memory, V from
 //                      shared memory); completion is signalled with tcgen05.commit.
 //   warps 0-3 / 4-7    softmax of head A / B, one thread per query row: tcgen05.ld of the 64 scores,
 //                      scales / masks, online softmax in base 2 with a lazily updated maximum (the O
@@ -22,7 +22,10 @@
 //                      2^8), P as bf16 pairs written back over the first 32 columns of the same S buffer,
 //                      final O / l from tensor memory.
 // Tensor memory (512 columns): S_A0 | S_A1 | S_B0 | S_B1 (64 each) | O_A | O_B (128 each).
-// All shared-memory operands are K-major: V is transposed once per call by the preparation pass.
+// Shared-memory operands are K-major, but for V of 16-bit P V where the caller gives it as it lies (v_rows): a tile is then two
+// boxes of 64 keys x 64 channels, an MN-major operand, and nothing is transposed or padded (keys past N load as zero).
+// With V transposed first, a call took 8 us more at 8K and 5 to 8 us of 105 at 2 x 1973; a plan that is kept for later and
+// FP8 P V (V is quantised anyway) still take V^T.
 // Every wait is bounded and abortable; a failed wait raises bit 1 of the status word, and the rows of the block and of
 // those after it are NaN.
 #include "hq_tc05.cuh"
@@ -36,6 +39,7 @@ struct PrefillTcParams {
   void* out; int out_dtype; int64_t o_sb, o_sh, o_sn;
   int B, H_Q, H_KV, N, Npad, W, T, Tpad, nqb, nkb;
   int group;                                       // head pairs whose blocks are launched together
+  int v_rows;                                      // V tiles are rows of keys (mVt 4-D, mXv 2-D) instead of V^T
   float sml;
   int* status;
 };
@@ -54,7 +58,7 @@ struct TcSmem {              // offsets from a 1024-aligned base
   static constexpr int Qi = 0;                             // 2 x 16 KB  [head][128 rows][128 B] int8
   static constexpr int Qb = 32768;                         // 2 x 32 KB  [head][2 halves][128 rows][128 B] bf16
   static constexpr int K = 98304;                          // kKStages x 16 KB: int8 tile, or two bf16 halves
-  static constexpr int V = K + kKStages * 16384;           // kVStages x 16 KB: V^T [128 d rows][128 B]
+  static constexpr int V = K + kKStages * 16384;           // kVStages x 16 KB: V^T [128 d rows][128 B], or V [2 halves of d][64 key rows][128 B]
   static constexpr int Ks = V + kVStages * 16384;          // kKsSlots x kKsBytes
   static constexpr int Bar = Ks + kKsSlots * kKsBytes;     // barriers + scratch
   static constexpr int Total = Bar + 256;
@@ -360,7 +364,12 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap mQi, const __grid_constant
           uint8_t* sV = smem + TcSmem::V + cv.stage * 16384;
           uint64_t* full = v_full + cv.stage;
           mbar_expect_tx(full, kFp8 ? 8192 : 16384);      // FP8: V^T tiles of 64 one-byte keys
-          if (cv.kind == 1) tc::tma_load_2d(sV, &mXv, cv.j * 64, (int)((bhq0 + cv.hh) * 128), full);
+          if (!kFp8 && p.v_rows) {            // two boxes of 64 channels
+            for (int x = 0; x < 2; ++x) {
+              if (cv.kind == 1) tc::tma_load_2d(sV + 8192 * x, &mXv, 64 * x, (int)((bhq0 + cv.hh) * p.Tpad + cv.j * 64), full);
+              else tc::tma_load_4d(sV + 8192 * x, &mVt, 64 * x, (cv.kind == 0 ? 0 : wla) + cv.j * 64, hkv, b, full);
+            }
+          } else if (cv.kind == 1) tc::tma_load_2d(sV, &mXv, cv.j * 64, (int)((bhq0 + cv.hh) * 128), full);
           else tc::tma_load_2d(sV, &mVt, (cv.kind == 0 ? 0 : wla) + cv.j * 64, (int)(bhk * 128), full);
           cv.next(plan);
           progress = true;
@@ -396,7 +405,8 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap mQi, const __grid_constant
     if (h < plan.nheads) {
       constexpr uint32_t idesc_i8 = tc::make_idesc(2, tc::kFmtS8, tc::kFmtS8, 128, 64);
       constexpr uint32_t idesc_qk = tc::make_idesc(1, tc::kFmtBF16, tc::kFmtBF16, 128, 64);
-      constexpr uint32_t idesc_pv = tc::make_idesc(1, tc::kFmtBF16, tc::kFmtBF16, 128, 128);
+      const uint32_t idesc_pv = tc::make_idesc(1, tc::kFmtBF16, tc::kFmtBF16, 128, 128) | (p.v_rows ? tc::kBMnMajor : 0u);
+      const uint32_t v_step = p.v_rows ? 2048 >> 4 : 32 >> 4;       // 16 keys, in units of the descriptor
       constexpr uint32_t idesc_pv8 = tc::make_idesc(1, tc::kFmtE4M3, tc::kFmtE4M3, 128, 128);
       auto wait = [&](uint64_t* bar, uint32_t par) { return mbar_wait_warp(bar, par, abort_flag); };
       bool ok = wait(q_full + (plan.n_rest > 0 ? 0 : 1), 0), q_bf = plan.n_rest == 0;
@@ -404,7 +414,8 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap mQi, const __grid_constant
       const uint64_t dQi = tc::smem_desc_k128(smem + TcSmem::Qi + h * 16384, 0);
       const uint64_t dQb = tc::smem_desc_k128(smem + TcSmem::Qb + h * 32768, 0);
       const uint64_t dK = tc::smem_desc_k128(smem + TcSmem::K, 0);
-      const uint64_t dV = kFp8 ? tc::smem_desc_k64(smem + TcSmem::V, 0) : tc::smem_desc_k128(smem + TcSmem::V, 0);
+      const uint64_t dV = kFp8 ? tc::smem_desc_k64(smem + TcSmem::V, 0)
+                               : p.v_rows ? tc::smem_desc_mn128(smem + TcSmem::V, 8192) : tc::smem_desc_k128(smem + TcSmem::V, 0);
       const uint32_t tS = tmem_base + kColS + 128u * h, tO = tmem_base + kColO + 128u * h;
       const int n_t = plan.n_tiles(h), n_rest = plan.n_rest;
       TcItemIter cq, cp;
@@ -436,7 +447,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap mQi, const __grid_constant
           for (int k = 0; k < 2; ++k) tc::mma_f8_ts(tO, aP + 8 * k, bV + 2 * k, idesc_pv8, (t > 0 || k > 0) ? 1u : 0u);
         } else {
 #pragma unroll
-          for (int k = 0; k < 4; ++k) tc::mma_bf16_ts(tO, aP + 8 * k, bV + 2 * k, idesc_pv, (t > 0 || k > 0) ? 1u : 0u);
+          for (int k = 0; k < 4; ++k) tc::mma_bf16_ts(tO, aP + 8 * k, bV + v_step * k, idesc_pv, (t > 0 || k > 0) ? 1u : 0u);
         }
         tc::mma_commit(pv_done + 2 * h + (t & 1));
         tc::mma_commit(v_empty + stage);
@@ -833,7 +844,8 @@ transpose_v_kernel(const __nv_bfloat16* __restrict__ v, int64_t sb, int64_t sh, 
   }
 }
 
-// gathered vertical rows: xk [B,H_Q,Tpad,128] (rows >= T zero), xvt [B,H_Q,128,Tpad] (transposed V rows)
+// gathered vertical rows: xk [B,H_Q,Tpad,128] (rows >= T zero), and of V xvt [B,H_Q,128,Tpad] (transposed), or as rows like xk
+template <bool kRows>
 __global__ void __launch_bounds__(256)
 vertical_gather_t_kernel(const int* __restrict__ vasc, int T, int Tpad, int N, int H_Q, int H_KV,
                          const __nv_bfloat16* __restrict__ k_bf,
@@ -852,10 +864,15 @@ vertical_gather_t_kernel(const int* __restrict__ vasc, int T, int Tpad, int N, i
       vr = __ldg(reinterpret_cast<const uint4*>(v + b * v_sb + hkv * v_sh + (int64_t)src * v_sn + c));
     }
     *reinterpret_cast<uint4*>(xk + (bhq * Tpad + j0 + r) * 128 + c) = kr;
+    if constexpr (kRows) {
+      *reinterpret_cast<uint4*>(xvt + (bhq * Tpad + j0 + r) * 128 + c) = vr;
+      continue;
+    }
     const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&vr);
 #pragma unroll
     for (int j = 0; j < 8; ++j) tile[r][c + j] = e[j];
   }
+  if constexpr (kRows) return;
   __syncthreads();
   for (int x = tid; x < 128 * 8; x += 256) {
     const int d = x >> 3, k8 = (x & 7) * 8;
@@ -866,7 +883,7 @@ vertical_gather_t_kernel(const int* __restrict__ vasc, int T, int Tpad, int N, i
   }
 }
 
-int prefill_tc_launch(const hq_prefill_args* a, cudaStream_t st) {
+int prefill_tc_launch(const hq_prefill_args* a, bool v_rows, cudaStream_t st) {
   const int N = a->N, Npad = (N + 63) / 64 * 64, T = a->T, Tpad = (T + 63) / 64 * 64;
   CUtensorMap mQi, mQb, mKi, mKb, mVt, mXk, mXv, mKs, mKbs;
   const uint64_t qrows = (uint64_t)a->B * a->H_Q * N, krows = (uint64_t)a->B * a->H_KV * N;
@@ -879,6 +896,8 @@ int prefill_tc_launch(const hq_prefill_args* a, cudaStream_t st) {
   if (fp8) {       // V^T as e4m3 bytes: 64-key tiles are 64-byte rows, 64-byte swizzle
     if ((rc = tc::make_map_2d(&mVt, a->v_t8, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, (uint64_t)Npad, (uint64_t)a->B * a->H_KV * 128,
                               (uint64_t)Npad, 64, 128, 64))) return rc;
+  } else if (v_rows) {
+    if ((rc = tc::make_map_v_rows(&mVt, a->v_t, a->B, a->H_KV, N, a->v_sb, a->v_sh, a->v_sn))) return rc;
   } else if ((rc = tc::make_map_2d(&mVt, a->v_t, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)Npad, (uint64_t)a->B * a->H_KV * 128,
                                    (uint64_t)Npad * 2, 64, 128))) return rc;
   if ((rc = tc::make_map_2d(&mKs, a->k_scale, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, (uint64_t)Npad, (uint64_t)a->B * a->H_KV,
@@ -890,6 +909,8 @@ int prefill_tc_launch(const hq_prefill_args* a, cudaStream_t st) {
     if (fp8) {
       if ((rc = tc::make_map_2d(&mXv, a->vert_vt8, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, (uint64_t)Tpad, (uint64_t)a->B * a->H_Q * 128,
                                 (uint64_t)Tpad, 64, 128, 64))) return rc;
+    } else if (v_rows) {
+      if ((rc = tc::make_map_2d(&mXv, a->vert_vt, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, 128, (uint64_t)a->B * a->H_Q * Tpad, 256, 64, 64))) return rc;
     } else if ((rc = tc::make_map_2d(&mXv, a->vert_vt, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)Tpad, (uint64_t)a->B * a->H_Q * 128,
                                      (uint64_t)Tpad * 2, 64, 128))) return rc;
   } else {
@@ -902,6 +923,7 @@ int prefill_tc_launch(const hq_prefill_args* a, cudaStream_t st) {
   p.B = a->B; p.H_Q = a->H_Q; p.H_KV = a->H_KV; p.N = N; p.Npad = Npad; p.W = a->window; p.T = T; p.Tpad = Tpad;
   p.nqb = (N + 127) / 128; p.nkb = (N + 63) / 64;
   p.sml = a->sm_scale * 1.44269504f;
+  p.v_rows = v_rows;
   p.status = a->status;
   const size_t smem = TcSmem::Total + 1024;
   static thread_local int attr_dev = -1;
@@ -1033,12 +1055,12 @@ int prefill_tc_prepare_v(const void* v, int64_t sb, int64_t sh, int64_t sn, int 
   return HQ_OK;
 }
 
-int prefill_tc_prepare_vertical(const int32_t* vasc, int B, int H_Q, int H_KV, int N, int T, const void* k_bf, const void* v,
+int prefill_tc_prepare_vertical(bool rows, const int32_t* vasc, int B, int H_Q, int H_KV, int N, int T, const void* k_bf, const void* v,
                                 int64_t v_sb, int64_t v_sh, int64_t v_sn, void* xk, void* xvt, cudaStream_t st) {
   const int Tpad = (T + 63) / 64 * 64;
-  vertical_gather_t_kernel<<<dim3(Tpad / 64, B * H_Q), 256, 0, st>>>(vasc, T, Tpad, N, H_Q, H_KV, (const __nv_bfloat16*)k_bf,
-                                                                    (const __nv_bfloat16*)v, v_sb, v_sh, v_sn,
-                                                                    (__nv_bfloat16*)xk, (__nv_bfloat16*)xvt);
+  const auto kernel = rows ? vertical_gather_t_kernel<true> : vertical_gather_t_kernel<false>;
+  kernel<<<dim3(Tpad / 64, B * H_Q), 256, 0, st>>>(vasc, T, Tpad, N, H_Q, H_KV, (const __nv_bfloat16*)k_bf, (const __nv_bfloat16*)v, v_sb,
+                                                   v_sh, v_sn, (__nv_bfloat16*)xk, (__nv_bfloat16*)xvt);
   HQ_CUDA(cudaGetLastError());
   return HQ_OK;
 }

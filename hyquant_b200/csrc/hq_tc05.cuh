@@ -49,6 +49,25 @@ inline int make_map_2d(CUtensorMap* m, const void* base, CUtensorMapDataType dt,
   return HQ_OK;
 }
 
+// V rows as they lie in memory: [B][H][N][128] bf16 with element strides, boxes of 64 channels x 64 keys, 128-byte swizzle; keys
+// past N read as zero.
+inline int make_map_v_rows(CUtensorMap* m, const void* base, uint64_t B, uint64_t H, uint64_t N, int64_t sb, int64_t sh, int64_t sn) {
+  EncodeTiledFn fn = encode_fn();
+  if (fn == nullptr) { set_error("cuTensorMapEncodeTiled is not available from this driver"); return HQ_ERR_CUDA; }
+  const cuuint64_t dims[4] = {128, N, H, B};
+  const cuuint64_t strides[3] = {(cuuint64_t)sn * 2, (cuuint64_t)sh * 2, (cuuint64_t)sb * 2};
+  const cuuint32_t box[4] = {64, 64, 1, 1}, estr[4] = {1, 1, 1, 1};
+  const CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) {
+    set_error("cuTensorMapEncodeTiled failed with %d (v rows, N=%llu, strides %lld %lld %lld)", (int)r, (unsigned long long)N,
+              (long long)sb, (long long)sh, (long long)sn);
+    return HQ_ERR_CUDA;
+  }
+  return HQ_OK;
+}
+
 #if defined(__CUDACC__)
 // ------------------------------------------------------------------ device: barriers
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
@@ -76,6 +95,13 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
           smem_u32(dst)),
       "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(x), "r"(y)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, int x, int y, int z, int w, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];" ::"r"(
+          smem_u32(dst)),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z), "r"(w)
       : "memory");
 }
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* map) {
@@ -174,10 +200,24 @@ __device__ __forceinline__ uint64_t smem_desc_k64(const void* tile, uint32_t k_b
   return d;
 }
 
+// The same for a tile whose rows run along K and are 128 bytes of the M or N extent each (MN-major, 128-byte swizzle): K in
+// groups of 8 rows 1024 bytes apart, the extent in parts of 128 bytes `part` bytes apart.  A step of 16 along K adds 2048
+// bytes to the start address.
+__device__ __forceinline__ uint64_t smem_desc_mn128(const void* tile, uint32_t part) {
+  uint64_t d = 0;
+  d |= (uint64_t)((smem_u32(tile) & 0x3FFFFu) >> 4);
+  d |= (uint64_t)(part >> 4) << 16;
+  d |= (uint64_t)(1024 >> 4) << 32;
+  d |= (uint64_t)1 << 46;
+  d |= (uint64_t)2 << 61;
+  return d;
+}
+
 // instruction descriptor: D format (1 = f32, 2 = s32), A/B element formats, K-major operands, M x N
 __host__ __device__ constexpr uint32_t make_idesc(uint32_t dfmt, uint32_t afmt, uint32_t bfmt, uint32_t M, uint32_t N) {
   return (dfmt << 4) | (afmt << 7) | (bfmt << 10) | ((N >> 3) << 17) | ((M >> 4) << 24);
 }
+constexpr uint32_t kBMnMajor = 1u << 16;      // B operand MN-major
 constexpr uint32_t kFmtBF16 = 1;   // kind::f16: 0 = f16, 1 = bf16
 constexpr uint32_t kFmtS8 = 1;     // kind::i8 : 0 = u8, 1 = s8
 constexpr uint32_t kFmtE4M3 = 0;   // kind::f8f6f4: 0 = e4m3, 1 = e5m2

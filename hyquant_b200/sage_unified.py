@@ -163,12 +163,16 @@ class PrefillPlan:
         vert_k = vert_vt = nvv = vasc = None
         Npad = (N + 63) // 64 * 64
         v_t = v_t8 = v_sc8 = None
+        # 16-bit P V reads V where it lies if the plan may keep an input; else, and for FP8, V is transposed first
+        v_rows = alias_inputs and not pv_fp8 and N > 0 and all(s >= 128 for s in vb.stride()[:3])
         if pv_fp8:
             v_t8 = torch.empty(B, H_kv, 128, Npad, dtype=torch.uint8, device=dev)
             v_sc8 = torch.empty(B, H_kv, 128, dtype=torch.float32, device=dev)
             scratch = torch.empty(B * H_kv * 128, dtype=torch.int32, device=dev)
             _lib.check(lib.hq_prefill_quant_v_fp8(vb.data_ptr(), vb.stride(0), vb.stride(1), vb.stride(2), B, H_kv, N,
                                                   v_t8.data_ptr(), v_sc8.data_ptr(), scratch.data_ptr(), st), "hq_prefill_quant_v_fp8")
+        elif v_rows:
+            v_t = vb
         else:
             v_t = torch.empty(B, H_kv, 128, Npad, dtype=torch.bfloat16, device=dev)
             _lib.check(lib.hq_prefill_transpose_v(vb.data_ptr(), vb.stride(0), vb.stride(1), vb.stride(2), B, H_kv, N,
@@ -188,14 +192,15 @@ class PrefillPlan:
                 vasc = vid.clamp(0, prefix_len - 1).sort(dim=-1).values.to(torch.int32).contiguous()   # reference :510
             Tpad = (T + 63) // 64 * 64
             vert_k = torch.empty(B, H_q, Tpad, 128, dtype=torch.bfloat16, device=dev)
-            vert_vt = torch.empty(B, H_q, 128, Tpad, dtype=torch.bfloat16, device=dev)
+            vert_vt = torch.empty((B, H_q, Tpad, 128) if v_rows else (B, H_q, 128, Tpad), dtype=torch.bfloat16, device=dev)
             nvv = torch.empty(B, H_q, nqb, dtype=torch.int32, device=dev)
         # per (query head, key) term of the INT8 score conversion; -inf on the head's vertical lines
         ptr = lambda t: None if t is None else t.data_ptr()     # noqa: E731
         k_bias = k_bf if bf16_only else torch.empty(B, H_q, Npad, dtype=torch.float32, device=dev)
-        rc = 0 if bf16_only else lib.hq_prefill_vertical_prepare(ptr(vasc), B, H_q, H_kv, N, window_size, T, k_bf.data_ptr(),
-                                             vb.data_ptr(), vb.stride(0), vb.stride(1), vb.stride(2), k_sc.data_ptr(),
-                                             ptr(vert_k), ptr(vert_vt), k_bias.data_ptr(), ptr(nvv), st)
+        prepare = lib.hq_prefill_vertical_prepare_rows if v_rows else lib.hq_prefill_vertical_prepare
+        rc = 0 if bf16_only else prepare(ptr(vasc), B, H_q, H_kv, N, window_size, T, k_bf.data_ptr(),
+                                         vb.data_ptr(), vb.stride(0), vb.stride(1), vb.stride(2), k_sc.data_ptr(),
+                                         ptr(vert_k), ptr(vert_vt), k_bias.data_ptr(), ptr(nvv), st)
         _lib.check(rc, "hq_prefill_vertical_prepare")
         vert_vt8 = None
         if pv_fp8 and T:
@@ -216,6 +221,8 @@ class PrefillPlan:
             a.v_t8, a.v_scale8, a.pv_fp8 = v_t8.data_ptr(), v_sc8.data_ptr(), 1
         else:
             a.v_t = v_t.data_ptr()
+            if v_rows:
+                a.v_rows, a.v_sb, a.v_sh, a.v_sn = 1, vb.stride(0), vb.stride(1), vb.stride(2)
         if T:
             a.vert_k, a.vert_vt, a.nv_valid = vert_k.data_ptr(), vert_vt.data_ptr(), nvv.data_ptr()
             if vert_vt8 is not None:

@@ -380,6 +380,12 @@ int hq_prefill_vertical_prepare(const int32_t* vidx_asc, int B, int H_Q, int H_K
                                 const float* k_scale, void* vert_k, void* vert_vt, float* k_bias, int32_t* nv_valid,
                                 void* stream);
 
+/* The same with the gathered rows of v as rows: vert_v bf16 [B,H_Q,Tpad,128], rows >= T zero (hq_prefill_args.v_rows). */
+int hq_prefill_vertical_prepare_rows(const int32_t* vidx_asc, int B, int H_Q, int H_KV, int N, int window, int T,
+                                     const void* k_bf, const void* v, int64_t v_sb, int64_t v_sh, int64_t v_sn,
+                                     const float* k_scale, void* vert_k, void* vert_v, float* k_bias, int32_t* nv_valid,
+                                     void* stream);
+
 /* V transposed for the K-major operands of the tensor-memory kernel (the job of the reference's
  * TransposePadPermuteKernel, vendor/sageattention/csrc/fused/fused.cu:264-315, without the fragment
  * permutation): v bf16 [B,H_KV,N,128] -> v_t bf16 [B,H_KV,128,Npad], columns >= N zero. */
@@ -416,8 +422,12 @@ typedef struct hq_prefill_args {
    *  csrc/qattn/attn_utils.cuh:30,354-458, csrc/qattn/qk_int_sv_f8_cuda_sm90.cu:259-364,490-515). v_t is not used then. */
   const void* v_t8;            /* e4m3 [B,H_KV,128,Npad] */
   const float* v_scale8;       /* fp32 [B,H_KV,128] */
-  int32_t pv_fp8; int32_t reserved0;
+  int32_t pv_fp8;
+  int32_t v_rows;              /* != 0 (16-bit P V only): v_t is V itself, bf16 rows [B,H_KV,N,128] with the strides below, and
+                                * vert_vt the rows [B,H_Q,Tpad,128] from hq_prefill_vertical_prepare_rows; nothing is transposed */
   const void* vert_vt8;        /* T > 0: e4m3 [B,H_Q,128,Tpad] from hq_prefill_vertical_gather_v_fp8 (vert_vt is not used then) */
+  int64_t v_sb, v_sh, v_sn;    /* v_rows: strides of V in elements, positive multiples of 8 (a struct that ends before them is
+                                * taken with v_rows == 0) */
 } hq_prefill_args;
 int hq_prefill_hybrid(const hq_prefill_args* args, void* stream);
 

@@ -331,3 +331,28 @@ def test_full_size_rows_against_fp32_reference():
         o = out[:, :, rows]
         assert (o - ref).abs().max().item() <= MAX_ABS
         assert ((o - ref) ** 2).sum().item() / (ref ** 2).sum().item() <= REL_MSE
+
+
+@pytest.mark.parametrize("B,H_Q,H_KV,N,W,T,layout", [(1, 4, 2, 64, 0, 0, "rows"), (2, 6, 2, 129, 64, 3, "rows"), (2, 4, 2, 1000, 128, 65, "tokens"),
+                                                     (1, 3, 1, 777, 777, 0, "tokens"), (2, 2, 2, 1, 1, 0, "rows"), (1, 8, 4, 515, 128, 64, "expanded")])
+def test_v_read_where_it_lies_equals_v_transposed(B, H_Q, H_KV, N, W, T, layout):
+    """The one-shot route takes V tiles as rows of keys (MN-major operands), a kept plan as V^T: the same products in the same
+    order, so the same bits - at ragged ends (keys past N are zero, not the next head's rows, which are NaN here), with V
+    strided by token, and with strides that only the transposed route takes."""
+    from hyquant_b200.sage_unified import PrefillPlan, hybrid_prefill
+    g = torch.Generator(device="cpu").manual_seed(N + T)
+    rnd = lambda *s: torch.randn(*s, generator=g).to(torch.bfloat16).cuda()     # noqa: E731
+    q, k, v = rnd(B, H_Q, N, 128), rnd(B, H_KV, N, 128), rnd(B, H_KV, N, 128)
+    if H_KV > 1 and layout != "expanded":
+        v[:, 1] = float("nan")
+    if layout == "tokens":
+        v = v.transpose(1, 2).contiguous().transpose(1, 2)
+    elif layout == "expanded":
+        v = v[:, :1].expand(B, H_KV, N, 128)
+    idx = torch.stack([torch.randperm(N - W, generator=g)[:T] for _ in range(B * H_Q)]).reshape(B, H_Q, T).cuda() if T else None
+    smooth = W < N
+    a = hybrid_prefill(q, k, v, idx, W, None, smooth)
+    b = PrefillPlan(q, k, v, idx, W, None, smooth).run()
+    head0 = a[:, :H_Q // H_KV]
+    assert bool(torch.isfinite(head0.float()).all())
+    assert torch.equal(a.view(torch.int16), b.view(torch.int16))

@@ -520,9 +520,8 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap mQi, const __grid_constant
         }
         for (; t < tq; ++t) {
           // the operands first, P last: from the moment P is there nothing is waited for, and P V of t and Q K^T of t + 2
-          // are issued together (a wait costs the warp some 400 clocks even if what it waits for is there: 32K hybrid
-          // 9.27 -> 9.05 ms, 8K 867 -> 844 us).  Not across a run of the other head's items: that head needs the V slots
-          // which P V of t and t + 1 give back to come to the end of its run, and K of t + 2 lies behind it - the two heads
+          // are issued together (32K hybrid 9.27 -> 9.05 ms, 8K 867 -> 844 us, while a wait cost the warp some 400 clocks).  Not
+          // across a run of the other head's items: that head needs the V slots which P V of t and t + 1 give back to come to the end of its run, and K of t + 2 lies behind it - the two heads
           // would wait for one another (with rings of three and four slots: runs of five items and more).
           const bool more = tq == t + 2 && tq < n_t && !run_ahead();
           v_ready();
@@ -654,10 +653,10 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap mQi, const __grid_constant
       for (; ok && t < n_rest && t < n_tiles; ++t) tile(t, TcTrue{});
       for (; ok && t < n_tiles; ++t) tile(t, TcFalse{});
     } else {
-      // (Asking for the next scores before the hand-over of P was measured slower here: 9.37 against 9.25 ms at 32K.  So were two
-      // threads per row, sixteen softmax warps in all: 10.1 ms - the loop lives on shared-memory bandwidth, of which
-      // the key scales and biases of 256 rows take 1024 clocks of some 2200 per pair of tiles and the operands of
-      // the products 640, and on the issuing warps' latency, which more warps lengthen.)
+      // The softmax warps pace the kernel: a tile's pass is some 1350 clocks with the other head's warp on the scheduler, 1050 alone
+      // (arithmetic 420, reads of scales and biases 256, exponentials 410, which a warp does not overlap).  Slower here: the next
+      // scores asked for before the hand-over of P; four rows x sixteen columns a thread (a third of the shared-memory
+      // wavefronts; 8K 650 to 685 us against 647); sixteen softmax warps, two threads per row or tiles taken in turn (773).
       float lim_sum = m_ref == -INFINITY ? -1.f : 256.f, mu = 0.f;      // a row without a reference: any sum calls for one
       auto tile = [&](int t, auto int8_tile) {
         constexpr bool is_i8 = decltype(int8_tile)::value;

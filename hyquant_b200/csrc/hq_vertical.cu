@@ -15,6 +15,7 @@
 // selected (key, ~index) pairs, the short distances inside warps.
 #include <cooperative_groups.h>
 #include "hq_common.cuh"
+#include "hq_topk_form.h"
 
 namespace hq {
 
@@ -196,7 +197,6 @@ __device__ __forceinline__ uint32_t orderable(float f) {
 }
 
 constexpr int kTopkThreads = 1024;
-constexpr int kTopkMaxK = 16384;
 
 __device__ __forceinline__ int block_exclusive_scan(int v, int* warp_sums, int& total) {
   // 1024 threads; returns exclusive prefix of v over the block, total in `total`
@@ -225,8 +225,6 @@ __device__ __forceinline__ int block_exclusive_scan(int v, int* warp_sums, int& 
   total = warp_sums[32];
   return warp_sums[warp] + inc - v;
 }
-
-constexpr int kTopkBins = 2048;
 
 // 64 entries per warp (lane l: base + l and base + 32 + l): the compare-exchange steps of a bitonic stage `size` whose
 // distance is at most `first` (32 or less), without leaving registers
@@ -378,7 +376,6 @@ topk_kernel(const float* __restrict__ scores, int64_t stride, int n, int k, int 
 
 // ---- the same for long rows
 constexpr int kSliceThreads = 512, kSliceWarps = kSliceThreads / 32;
-constexpr int kTopkCluster = 8;            // most blocks per row
 
 __device__ __forceinline__ int warp_inclusive_scan(int v) {
   const int lane = threadIdx.x & 31;
@@ -727,48 +724,34 @@ extern "C" int hq_topk(const float* scores, int64_t scores_stride, int rows, int
   HQ_REQUIRE(k <= n, HQ_ERR_INVALID, "hq_topk: k %d > n %d", k, n);
   HQ_REQUIRE(k <= kTopkMaxK, HQ_ERR_UNSUPPORTED, "hq_topk: k %d > %d", k, kTopkMaxK);
   HQ_REQUIRE(scores && idx_desc, HQ_ERR_INVALID, "hq_topk: null pointer");
-  int kpad = 64;
-  while (kpad < k) kpad <<= 1;
-  constexpr size_t kMaxSmem = 224 * 1024;
-  const size_t need = (size_t)kpad * 8 + kTopkBins * 4, with_keys = need + (size_t)n * 4;
   static thread_local int attr_dev = -1;
   int dev = 0;
   HQ_CUDA(cudaGetDevice(&dev));
   if (attr_dev != dev) {
-    HQ_CUDA(cudaFuncSetAttribute(topk_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem));
-    HQ_CUDA(cudaFuncSetAttribute(topk_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem));
-    HQ_CUDA(cudaFuncSetAttribute(topk_cluster_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem));
-    HQ_CUDA(cudaFuncSetAttribute(topk_cluster_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem));
+    HQ_CUDA(cudaFuncSetAttribute(topk_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTopkSmem));
+    HQ_CUDA(cudaFuncSetAttribute(topk_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTopkSmem));
+    HQ_CUDA(cudaFuncSetAttribute(topk_cluster_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTopkSmem));
+    HQ_CUDA(cudaFuncSetAttribute(topk_cluster_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTopkSmem));
     attr_dev = dev;
   }
-  // A cluster per row from 12K candidates on, with slices of 2K or more and no more blocks than two to an SM.  Measured (us, block /
-  // cluster): 8 or 32 rows of 8K 13.3 / 14.2, 64 of 16K 21.1 / 19.7 (four blocks; eight 25.3), 8 of 32K 36.3 / 19.2, 32 of 32K
-  // 36.4 / 23.4, 2 of 128K 146 / 41.
-  int blocks = kTopkCluster;
-  while (blocks > 1 && (n < 2048 * blocks || (int64_t)rows * blocks > 2 * sm_count())) blocks >>= 1;
-  if (n >= 12288 && blocks > 1) {
-    const int seg = ((n + blocks - 1) / blocks + 31) & ~31;
-    int selcap = 64;
-    while (selcap < (k < seg ? k : seg)) selcap <<= 1;
-    const size_t slice_need = (size_t)selcap * 8 + 2 * kTopkBins * 4, slice_keys = slice_need + (size_t)seg * 4;
+  const TopkForm f = topk_form(rows, n, k, sm_count());
+  if (f.blocks > 1) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)rows * blocks);
+    cfg.gridDim = dim3((unsigned)rows * f.blocks);
     cfg.blockDim = dim3(kSliceThreads);
-    cfg.dynamicSmemBytes = slice_keys <= kMaxSmem ? slice_keys : slice_need;
+    cfg.dynamicSmemBytes = f.smem;
     cfg.stream = (cudaStream_t)stream;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = (unsigned)blocks; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    at[0].val.clusterDim.x = (unsigned)f.blocks; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    if (slice_keys <= kMaxSmem) HQ_CUDA(cudaLaunchKernelEx(&cfg, topk_cluster_kernel<true>, scores, scores_stride, n, k, seg, selcap, idx_desc, idx_asc));
-    else HQ_CUDA(cudaLaunchKernelEx(&cfg, topk_cluster_kernel<false>, scores, scores_stride, n, k, seg, selcap, idx_desc, idx_asc));
+    const auto kernel = f.kept ? topk_cluster_kernel<true> : topk_cluster_kernel<false>;
+    HQ_CUDA(cudaLaunchKernelEx(&cfg, kernel, scores, scores_stride, n, k, f.seg, f.list, idx_desc, idx_asc));
     return HQ_OK;
   }
-  if (with_keys <= kMaxSmem)
-    topk_kernel<true><<<rows, kTopkThreads, with_keys, (cudaStream_t)stream>>>(scores, scores_stride, n, k, kpad, idx_desc, idx_asc);
-  else
-    topk_kernel<false><<<rows, kTopkThreads, need, (cudaStream_t)stream>>>(scores, scores_stride, n, k, kpad, idx_desc, idx_asc);
+  const auto kernel = f.kept ? topk_kernel<true> : topk_kernel<false>;
+  kernel<<<rows, kTopkThreads, f.smem, (cudaStream_t)stream>>>(scores, scores_stride, n, k, f.list, idx_desc, idx_asc);
   HQ_CUDA(cudaGetLastError());
   return HQ_OK;
 }

@@ -9,6 +9,7 @@ from hyquant_b200 import _lib
 from hyquant_b200.synth import gen_numpy
 from oracle import hq_oracle as orc
 from tests.helpers import load, max_abs, sha
+from tests.test_topk_form import form          # noqa: F401
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -89,8 +90,8 @@ def test_topk_exact_with_ties(n, k):
 
 @pytest.mark.parametrize("n,k", [(31, 5), (64, 64), (65, 64), (1025, 129), (53000, 2650), (56000, 100), (56300, 100), (60000, 16384)])
 def test_topk_edges_of_the_kept_row_and_the_warp_ranges(n, k):
-    """Rows that just fit the shared-memory copy of the keys and rows that do not, ranges of warps that are empty, lists
-    around the 64 entries a warp sorts by itself; infinities and a row of one value."""
+    """Ranges of warps that are empty, lists around the 64 entries a warp sorts by itself (a block a row up to 12K candidates,
+    then a cluster); infinities and a row of one value."""
     rng = np.random.Generator(np.random.PCG64(7 * n + k))
     s = rng.standard_normal((4, n), dtype=np.float32)
     s[1] = 0.25
@@ -184,8 +185,8 @@ def test_cache_reorganize_bit_exact(BH, N, W, T):
                                            (2, 32512, 1625, "one slice"), (70, 12301, 77, "normal"), (1, 131071, 6553, "normal"),
                                            (2, 40000, 9000, "infinities"), (1, 400001, 300, "normal")])
 def test_topk_of_long_rows(rows, n, k, kind):
-    """Rows that a cluster of blocks shares: odd slices, ties across slices, everything in one slice, lists too long to be
-    brought together, slices too long to be kept; the same list as the oracle's, bit for bit."""
+    """Long rows, few enough to be shared by clusters of blocks (but for 70 rows): odd slices, ties across slices, everything in
+    one slice, lists too long to be brought together; the same list as the oracle's, bit for bit."""
     rng = np.random.default_rng(n + k)
     s = rng.standard_normal((rows, n)).astype(np.float32)
     if kind == "ties":
@@ -197,6 +198,27 @@ def test_topk_of_long_rows(rows, n, k, kind):
         s[:, 5::1000] = np.inf
     idx, asc = hq.topk_indices(torch.from_numpy(s).to(DEV)[None], k, want_ascending=True)
     want = orc.topk_desc(s[None], k)
+    assert np.array_equal(idx.cpu().numpy(), want)
+    assert np.array_equal(asc.cpu().numpy(), np.sort(want, axis=-1))
+
+
+@pytest.mark.parametrize("rows,n,k,blocks,kept", [
+    (1, 440001, 300, 8, False),          # slices read again, lists brought together in the counters' place
+    (1, 200000, 10000, 8, False),        # slices read again, entries searched in the other blocks' lists
+    (20, 170000, 8500, 4, False), (20, 50000, 6300, 4, True), (37, 25000, 1250, 8, True), (64, 16400, 820, 4, True),
+    ("sms", 12500, 625, 1, True), ("sms", 46900, 2345, 1, True), ("sms", 57000, 2850, 1, False), (40, 60000, 16384, 1, False),
+    (75, 30000, 1500, 1, True)])
+def test_topk_in_every_form(form, rows, n, k, blocks, kept):      # noqa: F811
+    """Each kernel that the rule can pick, with ties across slices in every other row; "sms": a row more than the chip has SMs."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    rows = sms + 1 if rows == "sms" else rows
+    assert form(rows, n, k, sms)[0] == blocks and bool(form(rows, n, k, sms)[3]) == kept
+    rng = np.random.default_rng(rows + n)
+    s = rng.standard_normal((rows, n), dtype=np.float32)
+    s[1::2] = np.round(2 * s[1::2])
+    s[0, 100:] = np.where(s[0, 100:] > 0.5, np.float32(0.5), s[0, 100:])      # a plateau at the threshold
+    idx, asc = hq.topk_indices(torch.from_numpy(s).to(DEV), k, want_ascending=True)
+    want = orc.topk_desc(s, k)
     assert np.array_equal(idx.cpu().numpy(), want)
     assert np.array_equal(asc.cpu().numpy(), np.sort(want, axis=-1))
 

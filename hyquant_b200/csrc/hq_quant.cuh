@@ -43,72 +43,75 @@ __device__ __forceinline__ void load16(const float* p, float (&v)[16]) {
 // Returns the row's fp16 scale (the same on the row's eight lanes) and this lane's 16 codes packed in channel order
 // into `code` (BITS / 2 words: 16 bytes at 8 bits, 8 at 4, 4 at 2); a token row is 16 * BITS bytes and lane l owns
 // bytes [2 BITS (l & 7), 2 BITS ((l & 7) + 1)).
-// q = rint(x / sf) with the IEEE quotient without sixteen IEEE divisions per lane: the product with the correctly
-// rounded reciprocal is within 1.5 * 2^-23 (relative) of the rounded quotient, and |quotient| < 2^BITS, so the two round
-// to the same integer unless the product lies within kNearTie of a half-integer - only then the division is done
-// (quant_word, for the whole word).  Infinities and NaNs take the same values either way (x * 0 = x / inf = 0 or NaN
-// alike, inf * r = inf / sf).  NaN inputs: 0/0 cannot happen (the scale is >= half(1e-5 / q_max) > 0); inf / inf gives
-// NaN, which the clamp turns into the lowest code.
+// q = rint(x / sf), the IEEE quotient rounded half to even and clamped.  Infinities and NaNs: x / inf = 0; 0 / 0 cannot happen
+// (the scale is >= half(1e-5 / q_max) > 0); a NaN, inf / inf too, becomes the lowest code in the clamp.
 template <int BITS>
-__device__ __forceinline__ uint32_t quant_word(const float* x, float rcp, float sf) {
+__device__ __forceinline__ void quant_row16_exact(const float (&v)[16], float sf, uint32_t (&code)[BITS / 2]) {
   constexpr float qmax = (float)((1 << (BITS - 1)) - 1), qmin = -(float)(1 << (BITS - 1));
-  constexpr float kNearTie = BITS == 8 ? 1.5e-4f : 6e-6f;      // > 4 x the largest possible difference of the two
-  uint32_t c = 0;
+  constexpr int kPerWord = 32 / BITS;
 #pragma unroll
-  for (int i = 0; i < 32 / BITS; ++i) {
-    const float t = __fmul_rn(x[i], rcp);
-    float q = rintf(t);
-    if (0.5f - fabsf(t - q) < kNearTie) q = rintf(__fdiv_rn(x[i], sf));
-    q = fminf(fmaxf(q, qmin), qmax);
-    c |= ((uint32_t)(__float2int_rn(q)) & ((1u << BITS) - 1u)) << (BITS * i);
+  for (int w = 0; w < BITS / 2; ++w) {
+    uint32_t c = 0;
+#pragma unroll
+    for (int i = 0; i < kPerWord; ++i) {
+      const float q = fminf(fmaxf(rintf(__fdiv_rn(v[w * kPerWord + i], sf)), qmin), qmax);
+      c |= ((uint32_t)(__float2int_rn(q)) & ((1u << BITS) - 1u)) << (BITS * i);
+    }
+    code[w] = c;
   }
-  return c;
 }
 
-// The common word costs no conversion, clamp or mask: adding 1.5 * 2^23 rounds to the integer (ties to even, as rintf) and
-// leaves it in the low bits; shifted and added up, the sixteen codes plus 2^(BITS-1) each are digits without borrows, and
-// flipping their top bits makes them two's complement.  The largest distance from an integer is kept on the way (NaN stays);
-// a word with one near a tie, a NaN or an infinity, and rows whose scale is a subnormal half (only there can |x / sf| round past
-// q_max: a normal one is within 2^-11 of amax / q_max) go through quant_word.  With two conversions an element, and the two
-// searches of the reorganisation's blocks, 32K tokens of eight kv-heads took 73 us, 57 now (HBM floor 26).
+// The common row costs no division, conversion, clamp or mask, and the same whatever its values.  The product with the rounded
+// reciprocal, corrected once by its remainder (Markstein, IBM J. Res. Dev. 34, 1990), is on the same side of every half-integer
+// h as the IEEE quotient, and h where that is: h sf (19 bits at most) and the remainder are exact, so the quotient is h or at
+// least 2^-24 h away from it, at least 2^-43 h outside what rounds to h, and the corrected product is within 2^-46 h of it before its own
+// rounding.  Adding 1.5 * 2^23 rounds to the integer (ties to even, as rintf) and leaves it in the low bits; shifted and added up,
+// the sixteen codes plus 2^(BITS-1) each are digits without borrows, and flipping their top bits makes them two's complement.
+// The exact form takes lanes that hold a NaN, and rows whose scale is infinite or whose largest quotient rounds past q_max
+// (subnormal scales only: a normal one is within 2^-11 of amax / q_max); it stands inline, because an array handed to a
+// function is kept in local memory on the common path too (19 -> 31 us below).
+// 8 x 32K rows of bf16 that lie in L2, codes of 2 / 4 / 8 bits: 19 / 19 / 22 us, zero rows and half-integers the same.  With a
+// division instead wherever a product lies near a half-integer (bf16 rows often do in 2 bits) 31 / 25 / 22, half-integers
+// 42 / 38 / 55; the reorganisation of 32K tokens of eight kv-heads 57 us, now 44 (HBM floor 26).
 template <int BITS>
 __device__ __forceinline__ __half quant_row16(const float (&v)[16], int scale_mode, uint32_t (&code)[BITS / 2]) {
   constexpr float qmax = (float)((1 << (BITS - 1)) - 1);
-  float amax = 0.f;
+  float top = 0.f;
 #pragma unroll
-  for (int i = 0; i < 16; i += 2) amax = fmax3_abs(amax, v[i], v[i + 1]);
+  for (int i = 0; i < 16; i += 2) top = fmax3_abs_nan(top, v[i], v[i + 1]);
+  bool exact = top != top;
+  if (exact) {                                 // a NaN does not count for the scale
+    top = 0.f;
 #pragma unroll
-  for (int o = 4; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-  amax = fmaxf(amax, 1e-5f);
+    for (int i = 0; i < 16; i += 2) top = fmax3_abs(top, v[i], v[i + 1]);
+  }
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+  const float amax = fmaxf(top, 1e-5f);
   const float s32 = scale_mode == 0 ? __fdiv_rn(amax, qmax) : __fmul_rn(amax, __fdiv_rn(1.0f, qmax));
   const __half sh = __float2half_rn(s32);
   const float sf = __half2float(sh);
   const float rcp = __frcp_rn(sf);
-  constexpr float kNearTie = BITS == 8 ? 1.5e-4f : 6e-6f;
   constexpr int kPerWord = 32 / BITS;
   constexpr uint32_t kOnes = BITS == 8 ? 0x01010101u : BITS == 4 ? 0x11111111u : 0x55555555u;     // a one in every digit
   constexpr uint32_t kTop = kOnes << (BITS - 1);
   constexpr uint32_t kMagic = 0x4B400000u;                       // 1.5 * 2^23
-  const float2 rcp2 = make_float2(rcp, rcp), magic2 = make_float2(12582912.f, 12582912.f), unmagic2 = make_float2(-12582912.f, -12582912.f);
-  const bool tiny = !(sf >= 6.103515625e-05f);
+  const float2 rcp2 = make_float2(rcp, rcp), nsf2 = make_float2(-sf, -sf), magic2 = make_float2(12582912.f, 12582912.f);
 #pragma unroll
   for (int w = 0; w < BITS / 2; ++w) {
     uint32_t c = kTop - kMagic * kOnes;
-    float far = 0.f;
 #pragma unroll
     for (int i = 0; i < kPerWord; i += 2) {
-      const float2 t = fmul2(make_float2(v[w * kPerWord + i], v[w * kPerWord + i + 1]), rcp2);
-      const float2 r = fadd2(t, magic2);
-      const float2 q = fadd2(r, unmagic2);
-      const float2 d = ffma2(q, make_float2(-1.f, -1.f), t);
-      far = fmax3_abs_nan(far, d.x, d.y);
+      const float2 x = make_float2(v[w * kPerWord + i], v[w * kPerWord + i + 1]);
+      const float2 t = fmul2(x, rcp2);
+      const float2 r = fadd2(ffma2(ffma2(t, nsf2, x), rcp2, t), magic2);
       c += __float_as_uint(r.x) << (BITS * i);
       c += __float_as_uint(r.y) << (BITS * (i + 1));
     }
-    c ^= kTop;
-    if (tiny || !(0.5f - far >= kNearTie)) c = quant_word<BITS>(v + w * kPerWord, rcp, sf);
-    code[w] = c;
+    code[w] = c ^ kTop;
   }
+  exact |= !(rcp > 0.f && top * rcp < qmax + 0.499f);
+  if (__builtin_expect(exact, 0)) quant_row16_exact<BITS>(v, sf, code);
   return sh;
 }
 

@@ -250,7 +250,8 @@ def test_reorganisation_places_every_row(N, W, T, dense):
 @pytest.mark.parametrize("bits", [2, 4, 8])
 def test_quantiser_words_that_leave_the_common_path(bits):
     """Rows of subnormal scale (where a quotient can round past q_max), rows full of half-integers, and a NaN or an infinity in
-    one word of a row: the codes of the oracle; a NaN is the lowest code and does not count for the scale."""
+    one word of a row: the codes of the oracle; a NaN is the lowest code and does not count for the scale.  An infinite scale
+    (an infinity in the row, or a maximum past fp16) makes every finite value 0 and infinities the lowest code."""
     rng = np.random.default_rng(bits)
     qmax = 2 ** (bits - 1) - 1
     x = rng.standard_normal((1, 200, 128)).astype(np.float32)
@@ -273,3 +274,11 @@ def test_quantiser_words_that_leave_the_common_path(bits):
     want = clean.cpu().numpy().view(np.uint8).copy()
     want[0, :, 40 // per] |= low
     assert np.array_equal(got.cpu().numpy().view(np.uint8), want)
+    odd[0, 0, 40], odd[0, 1, 40] = np.inf, -np.inf
+    got, scale = hq.quantize_per_token(t_bf16(odd), bits)
+    want = np.zeros_like(want)
+    want[0, :, 40 // per] = low
+    assert bool(torch.isinf(scale).all()) and np.array_equal(got.cpu().numpy().view(np.uint8), want)
+    big = torch.randn(1, 3, 128, device=DEV) * torch.tensor([1e7, 1e20, 3e37], device=DEV)[None, :, None]
+    got, scale = hq.quantize_per_token(big, bits)
+    assert bool(torch.isinf(scale).all()) and not bool(got.any())

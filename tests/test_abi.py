@@ -39,6 +39,41 @@ def test_decode_args_struct_matches_header_size():
     assert b"struct_bytes" in _lib.lib().hq_last_error()
 
 
+def _prefill_args(**fields):
+    """Arguments of hq_prefill_hybrid that pass its checks up to the ones under test; the addresses are made up and never read."""
+    a = _lib.PrefillArgs()
+    a.struct_bytes = C.sizeof(_lib.PrefillArgs)
+    a.B, a.H_Q, a.H_KV, a.N, a.head_dim, a.window, a.T = 1, 2, 1, 256, 128, 64, 0
+    a.out_dtype, a.sm_scale = _lib.HQ_BF16, 0.1
+    for name in ("q_i8", "q_bf", "q_scale", "k_i8", "k_bf", "k_scale", "k_bias", "v_t", "out", "status"):
+        setattr(a, name, 1 << 20)
+    a.o_sb, a.o_sh, a.o_sn = 2 * 256 * 128, 256 * 128, 128
+    for name, value in fields.items():
+        setattr(a, name, value)
+    return a
+
+
+def test_prefill_args_struct_sizes():
+    """The struct as it is and as it ended before V's strides are taken; any other size is refused."""
+    lib = _lib.lib()
+    short = _lib.PrefillArgs.v_sb.offset
+    for size in (short, C.sizeof(_lib.PrefillArgs)):
+        assert lib.hq_prefill_hybrid(C.byref(_prefill_args(struct_bytes=size, head_dim=64)), None) == -2
+        assert b"head_dim" in lib.hq_last_error()                             # past the size check
+    for size in (0, short - 8, short + 8, short + 16, C.sizeof(_lib.PrefillArgs) + 8):
+        assert lib.hq_prefill_hybrid(C.byref(_prefill_args(struct_bytes=size)), None) == -1
+        assert b"struct_bytes" in lib.hq_last_error()
+
+
+@pytest.mark.parametrize("strides", [(0, 128, 128), (32768, 0, 128), (32768, 32768, 0), (-32768, 128, 128), (32768, 32768, 129), (32768, 132, 128),
+                                     (32772, 128, 128)])
+def test_prefill_rows_of_v_must_be_sixteen_bytes_apart(strides):
+    lib = _lib.lib()
+    a = _prefill_args(v_rows=1, v_sb=strides[0], v_sh=strides[1], v_sn=strides[2])
+    assert lib.hq_prefill_hybrid(C.byref(a), None) == -3
+    assert b"rows of v" in lib.hq_last_error()
+
+
 def test_argument_validation_without_gpu():
     lib = _lib.lib()
     n = C.c_int64(0)

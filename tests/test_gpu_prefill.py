@@ -353,6 +353,9 @@ def test_v_read_where_it_lies_equals_v_transposed(B, H_Q, H_KV, N, W, T, layout)
     smooth = W < N
     a = hybrid_prefill(q, k, v, idx, W, None, smooth)
     b = PrefillPlan(q, k, v, idx, W, None, smooth).run()
+    plan = PrefillPlan(q, k, v, idx, W, None, smooth)
+    plan.args.struct_bytes, plan.args.v_rows = type(plan.args).v_sb.offset, 7          # the struct before V's strides: the flag is not read
+    assert torch.equal(plan.run().view(torch.int16), b.view(torch.int16))
     head0 = a[:, :H_Q // H_KV]
     assert bool(torch.isfinite(head0.float()).all())
     assert torch.equal(a.view(torch.int16), b.view(torch.int16))

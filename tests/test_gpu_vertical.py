@@ -247,6 +247,30 @@ def test_reorganisation_places_every_row(N, W, T, dense):
             assert torch.equal(packed[h].view(torch.int8), codes[0]) and torch.equal(scale[h].reshape(-1), sc[0])
 
 
+@pytest.mark.parametrize("N,positions", [(700, [5] * 3 + [40, 41, 41, 127, 127, 128, 128, 128, 300]), (700, [130] * 200 + list(range(140, 200))), (300, [0, 0, 255, 255])])
+def test_reorganisation_with_positions_given_more_than_once(N, positions):
+    """A list that repeats positions (within a tile, across a tile's edge, more entries than a tile has rows): every entry counts
+    for the rows behind it, so that row p stands at p minus the entries below it; where two rows meet, either may stand."""
+    g = torch.Generator(device="cpu").manual_seed(N)
+    W, T = 44, len(positions)
+    kv = torch.randn(2, 1, 1, N, 128, generator=g).to(torch.bfloat16).to(DEV)
+    layer = hq.DStageLayerCache(0, k_bits=4, v_bits=2, window_size=W, use_vert=False)
+    layer.update_prefill(kv[0], kv[1])
+    layer.freeze(1, vertical_indices=torch.tensor(positions)[None, None].to(DEV))
+    sources = {}
+    for p in range(N - W):
+        at = p - sum(x < p for x in positions)
+        if p not in positions and 0 <= at < N - W - T:
+            sources.setdefault(at, []).append(p)
+    alone = {at: ps[0] for at, ps in sources.items() if len(ps) == 1}
+    assert len(alone) >= (N - W - T) // 4
+    at, ps = torch.tensor(list(alone)).to(DEV), torch.tensor(list(alone.values())).to(DEV)
+    for x, bits, packed, scale, topk in ((kv[0], 4, layer.k_quant_packed, layer.k_scale, layer.k_topk), (kv[1], 2, layer.v_quant_packed, layer.v_scale, layer.v_topk)):
+        codes, sc = hq.quantize_per_token(x[0, :, ps], bits)
+        assert torch.equal(packed[0, at].view(torch.int8), codes[0]) and torch.equal(scale[0, at], sc[0])
+        assert torch.equal(topk[0], x[0, 0, torch.tensor(positions).to(DEV)])
+
+
 @pytest.mark.parametrize("bits", [2, 4, 8])
 def test_quantiser_words_that_leave_the_common_path(bits):
     """Rows of subnormal scale (where a quotient can round past q_max), rows full of half-integers, and a NaN or an infinity in

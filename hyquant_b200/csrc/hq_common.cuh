@@ -124,7 +124,6 @@ __device__ __forceinline__ float2 fmul2(float2 a, float2 b) {
       : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)));
   return d;
 }
-// a + b rounded towards zero
 // max(a, |b|, |c|) for a >= 0; the second form returns NaN if any of the three is one, the first passes over them
 __device__ __forceinline__ float fmax3_abs(float a, float b, float c) {
   float d;
@@ -136,6 +135,7 @@ __device__ __forceinline__ float fmax3_abs_nan(float a, float b, float c) {
   asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
   return d;
 }
+// a + b rounded towards zero
 __device__ __forceinline__ float2 fadd2_rz(float2 a, float2 b) {
   float2 d;
   asm("add.rz.f32x2 %0, %1, %2;" : "=l"(*reinterpret_cast<unsigned long long*>(&d))

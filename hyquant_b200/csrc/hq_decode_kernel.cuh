@@ -252,8 +252,8 @@ __device__ __forceinline__ float group_sum(float v) {
 }
 
 // The rest of a unit's wait, out of line: the loops over units stay straight-line code where the data are there at the first
-// poll.  With the groups' maxima taken only where they are needed (below): two-tile 128K x 4 54.5 -> 52.0 us, batch 16
-// 120 -> 113, 32K 14.7 -> 14.3 (the maxima alone 53.7, 114, 14.4).
+// poll.  With the groups' maxima taken only where they are needed (below), calls back to back over several caches: two-tile
+// 128K x 4 54.5 -> 52.0 us, batch 16 120 -> 113, 32K 14.7 -> 14.3 (the maxima alone 53.7, 114, 14.4).
 static __device__ __noinline__ bool unit_wait_rest(uint64_t* bar, uint32_t parity) { return mbar_wait_bounded(bar, parity); }
 
 // Online-softmax bookkeeping shared by both unit kinds.  `mx` is the maximum of this thread's new scores of its two heads of

@@ -764,10 +764,11 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap mQi, const __grid_constant
       ok = __all_sync(0xffffffffu, tc::mbar_wait_abortable(pv_done + 2 * h + ((n_tiles - 1) & 1), (uint32_t)(((n_tiles - 1) >> 1) & 1), abort_flag));
     if (ok && n_tiles > 0) {
       tc::fence_after_sync();
-      // A thread holds a row, a store wants a row on neighbouring lanes: 16-bit outputs pass through the head's part of the
+      // A thread holds a row, a store wants a row on neighbouring lanes: BF16 outputs pass through the head's part of the
       // query buffer (its last product is done), sixteen-byte pieces permuted within a row so that neither side meets a
       // bank twice.  Written straight from the row's thread, a store instruction touched 32 rows: 4900
-      // clocks a block, now 3400.  (With the start above: 16-bit 2 x 1973 105 -> 101 us per call.)
+      // clocks a block, now 3400.  (With the start above: 16-bit 2 x 1973 107 -> 104 us per call.)  FP16 and FP32 outputs are
+      // written from the row's thread.
       const float inv = l > 0.f ? 1.f / l : 0.f;
       const float* vsc = kFp8 ? p.v_scale + bhk * 128 : nullptr;        // FP8 P V: the channel scales of V come back here
       const int hq = (int)(bhq - (int64_t)b * p.H_Q);
@@ -935,7 +936,7 @@ int prefill_tc_launch(const hq_prefill_args* a, bool v_rows, cudaStream_t st) {
   }
   const int R = a->H_Q / a->H_KV;
   const int pairs = (R + 1) / 2;                                  // two query heads of a KV group per CTA
-  // 32 MB of operands (INT8 K, BF16 V^T: 384 bytes a key) per group: an even finish needs a few hundred blocks in the last
+  // 32 MB of operands (INT8 K, BF16 V: 384 bytes a key) per group: an even finish needs a few hundred blocks in the last
   // group, which 24 to 64 MB all give
   const int64_t in_l2 = (32ll << 20) / ((int64_t)N * 384);
   const int kv_heads = a->B * a->H_KV;

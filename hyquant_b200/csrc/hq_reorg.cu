@@ -4,8 +4,8 @@
 // writes INT4 codes + scales for the kept prefix rows, BF16 copies of the
 // vertical-line rows and of the window.  The reference's
 // scatter(-1)/sort/gather chain becomes: for source position p, rank(p) =
-// number of vertical rows below p (looked up in the ascending index list, a
-// per-tile slice of which sits in shared memory); p is dropped if it is itself
+// number of vertical rows below p (the tile's place in the ascending index
+// list, and the bits of the tile's vertical rows in shared memory); p is dropped if it is itself
 // vertical, else it lands at row p - rank(p) of the compact prefix, quantised
 // on the way by the same warp-level routine the staging flush uses.
 #include "hq_quant.cuh"
@@ -69,7 +69,7 @@ cache_reorg_kernel(const __nv_bfloat16* __restrict__ keys, const __nv_bfloat16* 
     }
     if (threadIdx.x < kReorgTile / 32) s_bits[threadIdx.x] = 0u;
     __syncthreads();
-    const int lo = s_range[0], cnt = s_range[1] - lo;   // cnt <= rows in tile (indices are distinct)
+    const int lo = s_range[0], cnt = s_range[1] - lo;   // cnt <= rows in tile if the positions are distinct
     for (int i = threadIdx.x; i < cnt; i += blockDim.x) {
       const unsigned o = (unsigned)(__ldg(asc + lo + i) - p0);
       if (o < kReorgTile) atomicOr(&s_bits[o >> 5], 1u << (o & 31));

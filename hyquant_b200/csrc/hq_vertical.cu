@@ -9,10 +9,11 @@
 // K fragments come straight from global memory as 16-byte loads; the channel
 // axis is permuted consistently on both operands so that no shuffle is needed.
 //
-// Top-k kernel — latency-bound, one CTA per row (8 to 32 rows of a call): the row's keys are read once, eight loads a
-// thread in flight, and kept in shared memory; three-pass radix select of the k-th largest key with a scan over the
-// bins, order-preserving compaction (ties go to the lower index; it is also the ascending list), bitonic sort of the
-// selected (key, ~index) pairs, the short distances inside warps.
+// Top-k kernels — latency-bound: a row's keys are read once, eight loads a thread in flight, and kept in shared memory
+// where they fit; three-pass radix select of the k-th largest key with a scan over the bins, order-preserving
+// compaction (ties go to the lower index; it is also the ascending list), bitonic sort of the selected (key, ~index)
+// pairs, the short distances inside warps.  topk_kernel: one CTA per row.  topk_cluster_kernel: a cluster of four or
+// eight CTAs per row, for long rows of calls that leave SMs idle otherwise (the rule is in hq_topk_form.h).
 #include <cooperative_groups.h>
 #include "hq_common.cuh"
 #include "hq_topk_form.h"
@@ -243,8 +244,8 @@ __device__ __forceinline__ void bitonic_in_warp(unsigned long long& a, unsigned 
   }
 }
 
-// kCached: the row's keys stay in shared memory after the first pass (rows of up to some 50 thousand candidates);
-// longer rows read them again from L2.
+// kCached: the row's keys stay in shared memory after the first pass (with the list of kpad entries they have to fit 224 KB:
+// 55 thousand candidates with a list of 64, 22 thousand with 16384); longer rows read them again from L2.
 template <bool kCached>
 __global__ void __launch_bounds__(kTopkThreads)
 topk_kernel(const float* __restrict__ scores, int64_t stride, int n, int k, int kpad,
@@ -405,7 +406,8 @@ __device__ __forceinline__ int slice_exclusive_scan(int v, int* warp_sums) {
 // above the threshold (and its share of what equals it) in index order, sorts that, and an entry's place in the whole list
 // is its own plus, for every other block, the entries above it there (a binary search).  8 rows of 32K candidates: 36 us
 // with a block each (counting 20 K clocks, compaction 14 K, the sort 18 K of 74 K), 19 us this way.
-// kCached: the slice's keys stay in shared memory after the first pass (up to some 50 thousand); longer slices are read again.
+// kCached: the slice's keys stay in shared memory after the first pass, where seg keys, selcap entries and the counters fit 224 KB
+// (53 thousand keys with a list of 64, 36 thousand with 8192, 20 thousand with 16384); longer slices are read again.
 template <bool kCached>
 __global__ void __launch_bounds__(kSliceThreads)
 topk_cluster_kernel(const float* __restrict__ scores, int64_t stride, int n, int k, int seg, int selcap,
@@ -589,8 +591,8 @@ topk_cluster_kernel(const float* __restrict__ scores, int64_t stride, int n, int
   }
 
   // ---- places: entries are distinct (the index is part of them), so the lists of the blocks interleave without ties.  All
-  // lists are brought over where the counters and keys, which are done with, leave room for them (k of up to an eighth of
-  // the row's slices and 2048 besides), and the searches of an entry run side by side.
+  // lists are brought over where the counters and keys, which are done with, leave room for them (k up to 2048, and half a
+  // slice besides where its keys were kept), and the searches of an entry run side by side.
   cluster.sync();
   if (blocks > 1 && (size_t)k * 8 <= 2 * kTopkBins * sizeof(int) + (kCached ? (size_t)seg * 4 : 0)) {
     unsigned long long* all = reinterpret_cast<unsigned long long*>(hist);

@@ -6,7 +6,7 @@ tcgen05 / tensor-memory kernel (``hq_prefill_hybrid``) after one operand-prepara
 
 By design nothing is expanded to query heads and nothing is physically reordered:
 K/V stay at kv-head granularity, the vertical lines of a query head are removed from
-its INT8 pass by a bit mask and served from a small gathered BF16 copy.
+its INT8 pass by -inf in the head's bias row and served from a small gathered BF16 copy.
 """
 
 from __future__ import annotations
